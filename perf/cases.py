@@ -247,3 +247,110 @@ def tolerance(case):
     if kind == "head":
         return {"rel": 1e-4, "differ": 0.0}
     return {"rel": 1e-4}
+
+
+# ------------------------------------------------------------------------- the same in 64 bits
+_IQ4_NL = (-127, -104, -83, -65, -49, -35, -22, -10, 1, 13, 25, 38, 53, 69, 89, 113)
+
+
+def _nibbles(b):
+    return b & 15, b >> 4
+
+
+def _scales_k4(s):
+    """The eight 6-bit scales and minimums of [blocks, 12] bytes."""
+    lo, hi, top = s[:, 0:4], s[:, 4:8], s[:, 8:12]
+    return (torch.cat([lo & 63, (top & 15) | (lo >> 6 << 4)], 1), torch.cat([hi & 63, (top >> 4) | (hi >> 6 << 4)], 1))
+
+
+def _wide_blocks(t, raw):
+    """GGUF blocks [blocks, bytes] -> their weights [blocks, elements] in f64."""
+    def half(at):
+        return raw[:, at:at + 2].contiguous().view(torch.float16).double()
+
+    nb, b = raw.shape[0], raw.int()
+    if t == 8:
+        return half(0) * raw[:, 2:34].contiguous().view(torch.int8).double()
+    if t == 20:
+        lo, hi = _nibbles(b[:, 2:18])
+        table = torch.tensor(_IQ4_NL, dtype=torch.float64, device=raw.device)
+        return half(0) * table[torch.cat([lo, hi], 1).long()]
+    if t in (12, 13):
+        sc, mn = (v.double() for v in _scales_k4(b[:, 4:16]))
+        lo, hi = _nibbles(b[:, -128:].reshape(nb, 4, 32))
+        q = torch.stack([lo, hi], 2).reshape(nb, 8, 32)
+        if t == 13:  # sub-block g's fifth bits are bit g of the 32 qh bytes
+            bits = torch.arange(8, device=raw.device, dtype=torch.int32).view(1, 8, 1)
+            q = q + ((b[:, 16:48].unsqueeze(1) >> bits & 1) << 4)
+        return ((half(0) * sc).unsqueeze(2) * q.double() - (half(2) * mn).unsqueeze(2)).reshape(nb, 256)
+    lo, hi = _nibbles(b[:, :128].reshape(nb, 2, 64))
+    ql = torch.cat([lo, hi], 2).reshape(nb, 2, 4, 32)
+    shift = torch.arange(0, 8, 2, device=raw.device, dtype=torch.int32).view(1, 1, 4, 1)
+    q = (ql | (b[:, 128:192].reshape(nb, 2, 1, 32) >> shift & 3) << 4) - 32
+    sc = raw[:, 192:208].contiguous().view(torch.int8).double() * half(208)
+    return (sc.unsqueeze(2) * q.reshape(nb, 16, 16).double()).reshape(nb, 256)
+
+
+class _Wide:
+    def __init__(self, raw, t, out_dim, in_dim):
+        self.t, self.n, self.k = t, out_dim, in_dim
+        self.raw = raw.view(out_dim, -1)
+
+    def rows(self, at, count):
+        return _wide_blocks(self.t, self.raw[at:at + count].reshape(-1, BLOCK[self.t][0])).view(-1, self.k)
+
+    def mul(self, x, add=0.0):
+        step = max(1, (1 << 26) // self.k)
+        return torch.cat([x.double() @ self.rows(at, step).T for at in range(0, self.n, step)], 1) + add
+
+
+class _WideMaker(_Maker):
+    def device(self, t, out_dim, in_dim):
+        return _Wide(self.raw(t, out_dim, in_dim), t, out_dim, in_dim)
+
+    host = device
+
+
+def exact(case, seed):
+    mk, kind = _WideMaker(seed), case["kind"]
+
+    def normed(x, w):
+        x = x.double()
+        return x * (x.square().mean(1, keepdim=True) + 1e-6).rsqrt() * w.double()
+
+    if kind == "gemv":
+        n, k, b = case["out"], case["in"], case["batch"]
+        w, x = mk.device(TYPES[case["type"]], n, k), mk.rows(b, k)
+        return w.mul(x, {"none": lambda: 0.0, "bias": lambda: mk.rows(n), "residual": lambda: mk.rows(b, n)}[case["addend"]]())
+    if kind in ("layer", "runner"):
+        h, kv, f, b = case["hidden"], case["kv"], case["ffn"], case["batch"]
+        ta, tu, td = TYPES[case["attn"]], TYPES[case["up"]], TYPES[case["down"]]
+        if kind == "layer":
+            x = mk.rows(b, h)
+            wo, wd = mk.device(ta, h, h), mk.device(td, h, f)
+            wq, nq = [mk.device(ta, n, h) for n in (h, kv, kv)], mk.norm(h)
+            wu, nu = [mk.device(tu, f, h) for _ in range(2)], mk.norm(h)
+            q, k, v = [w.mul(normed(x, nq)) for w in wq]
+            mid = wo.mul(q, x)
+            gate, up = [w.mul(normed(mid, nu)) for w in wu]
+            return q, k, v, mid, gate, up, wd.mul(gate * torch.sigmoid(gate) * up, mid)
+        names = ("q", "k", "v", "o", "gate", "up", "down")
+        ws = [mk.host(t, n, k) for t, n, k in ((ta, h, h), (ta, kv, h), (ta, kv, h), (ta, h, h), (tu, f, h), (tu, f, h), (td, h, f))]
+        rows = {name: mk.rows(b, n) for name, n in (("x", h), ("attn", h), ("mid", h), ("act", f))}
+        src = ("x", "x", "x", "attn", "mid", "mid", "act")
+        add = {"o": rows["x"], "down": rows["mid"]}
+        return {name: w.mul(rows[s], add.get(name, 0.0)) for name, w, s in zip(names, ws, src)}
+    if kind == "head":
+        w, x = mk.device(TYPES[case["type"]], case["vocab"], case["dim"]), mk.rows(case["batch"], case["dim"])
+        if case["top"] == 2:
+            return None, w.mul(x).topk(2, 1).values
+        return None, w.mul(normed(x, mk.norm(case["dim"]))).amax(1), None  # indices: whole values
+    if kind == "prefill":
+        w = mk.device(TYPES[case["type"]], case["n"], case["k"])
+        return w.mul(mk.rows(case["m"], case["k"]).to(torch.bfloat16))
+    if kind == "dequant":
+        w = mk.device(TYPES[case["type"]], case["out"], case["in"])
+        return w.rows(0, w.n)
+    w = mk.host(TYPES[case["type"]], case["out"], case["in"])
+    x = mk.rows(case["batch"], case["in"])
+    return w.mul(x, mk.rows(case["out"])).reshape(-1)
