@@ -93,8 +93,8 @@ int cogni_qmm_set_kernel_choice(int choice) {
     gemm_prefill_set_split(choice - 52);
     return COGNI_QMM_OK;
   }
-  if (choice == 59) {  // prefill split along K: four ordered splits wherever allowed
-    gemm_prefill_set_split(3);
+  if (choice == 59 || choice == 69) {  // prefill split along K: four / eight parts wherever allowed
+    gemm_prefill_set_split(choice == 59 ? 3 : 4);
     return COGNI_QMM_OK;
   }
   if (choice >= 27 && choice <= 30) {  // at least 1 .. 4 column ranges per row of the tiled GEMV

@@ -25,7 +25,7 @@
 //     one 128-byte segment.
 // mbarrier rings decouple the three roles.  Every wait is bounded (tma_pipe.cuh).
 #include <cuda.h>
-#include <mutex>
+#include <atomic>
 #include <cuda_bf16.h>
 
 #include "qmm_common.cuh"
@@ -104,9 +104,8 @@ struct GemmParams {
   const uint8_t *w;
   void *y;
   int m_rows, n_out, k_in, out_bf16;
-  int ks_per_split;  // k-steps per blockIdx.z; with two splits the partial tiles are added onto a zeroed y
-  int splits;
-  unsigned *turns;   // four splits: [tile][4] turn counters that order the partial tiles' additions (else nullptr)
+  int ks_per_split;  // k-steps per blockIdx.z
+  int splits;        // CTAs of a cluster that share a tile along K (1: no cluster)
   long long row_bytes;
 };
 
@@ -675,30 +674,25 @@ __device__ __forceinline__ void expand_kstep(const Raw<TYPE> &raw, int ks, int h
   }
 }
 
-// Ordered split along K.  Four CTAs of a tile take a quarter of K each and add their partial tiles
-// into y (the first part of every group is stored, so y is not zeroed).  Float addition does not commute over four addends, so the order is fixed: the
-// tile's columns form four groups, split z adds its part of group (z + t) mod 4 at step t, and a
-// turn counter per (tile, group) admits the steps in order; in every step the four splits work on
-// different groups.  The order depends on the group only, so every launch gives the same bits.
-// The four CTAs of a tile must run at the same time: the host uses this only for grids of at most
-// one CTA per SM.  The wait is bounded like every wait.
-__device__ unsigned g_prefill_turns[8][64 * 4];  // [stream slot][tile][group], zero between launches
-
-__device__ __forceinline__ void wait_turn(const unsigned *turn, unsigned want) {
-  const unsigned long long t0 = global_ns();
-  for (unsigned spin = 0;; spin++) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(turn) : "memory");
-    if (v == want) return;
-    __nanosleep(64);
-    if ((spin & 63u) == 63u) {
-      if (pipe_broken()) return;
-      if (global_ns() - t0 > kPipeWaitLimitNs) {
-        atomicAdd(&g_pipe_wait_timeouts, 1u);
-        return;
-      }
-    }
-  }
+// Split along K.  The CTAs of a cluster (1 x 1 x splits) take an equal part of K of one tile each.
+// Every CTA leaves its partial tile in its own shared memory (the ring is idle by then), and each
+// adds up its share of the columns from all of them, in the order of the parts, through distributed
+// shared memory: the same bits launch after launch, nothing to zero, no atomics, and a bf16 y is
+// rounded once like an unsplit one.
+__device__ __forceinline__ uint32_t peer_smem(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float4 ld_peer4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void split_sync() {  // all threads of all CTAs of the cluster
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // ---------------------------------------------------------------------------- the kernel
@@ -864,29 +858,45 @@ __global__ void __launch_bounds__(threads_for(TYPE, STAGED, BN), 1)
     if constexpr (STAGED) {
       const int sb0 = ks0 >> 2;
       const int rr = min(r + n0 - raw_n0, kBM - 1);  // this thread's row of the raw box
-      for (int ks = 0; ks < nks; ks++) {
-        const int s = ks % kStages;
+      // 128-token tiles are bound by the expansion, a chain of latencies per k-step (wait, fetch,
+      // convert, store, proxy fence, arrive).  With eight dequant warps two k-steps at a time share
+      // the waits and the fence and their conversions overlap: one wave at in_dim 4096, us, Q6_K
+      // 47.8 -> 44.7, IQ4_NL 44.4 -> 40.6.  Not with sixteen (Q4_K 34.5 -> 35.5), nor where only two
+      // or three stages fit and the tensor cores would wait for the pair (256 tokens, Q4_K 38.6 ->
+      // 49.8, IQ4_NL 45.7 -> 53.6).
+      constexpr int kBatch = BN == 128 && kDequantWarps == 8 ? 2 : 1;
+      for (int ks = 0; ks < nks; ks += kBatch) {  // nks is a multiple of four
         const int sbl = ks >> 2, buf = sbl & 1;
         if ((ks & 3) == 0) mbar_wait(smem_u32(&raw_bars[buf]), (sbl >> 1) & 1);
-        if constexpr (kQuarter)
-          fetch_quarter_from<TYPE>(raw_win + buf * kRawStage + rr * Sb<TYPE>::bytes, (ks0 + ks) & 3, q2, cur[0]);
-        else if constexpr (TYPE == kQ6_K)
-          fetch_staged_q6<kHalves>(raw_win + buf * kRawStage, rr,
-                                   210 * (sb0 + sbl) - q6_window_start(sb0 + sbl, (int)p.row_bytes),
-                                   (ks0 + ks) & 3, h0, cur);
-        else  // the block of row r sits at r * block bytes: the global fetch code reads it as it is
-          fetch_raw_from<TYPE>(raw_win + buf * kRawStage + rr * Sb<TYPE>::bytes, (ks0 + ks) & 3, h0, cur[0]);
-        if ((ks & 3) == 3 || ks == nks - 1) {  // this warp has read all it needs of the window
+        Raw<TYPE> raws[kBatch][kHalves];
+#pragma unroll
+        for (int u = 0; u < kBatch; u++) {
+          const int j = (ks0 + ks + u) & 3;
+          if constexpr (kQuarter)
+            fetch_quarter_from<TYPE>(raw_win + buf * kRawStage + rr * Sb<TYPE>::bytes, j, q2, cur[0]);
+          else if constexpr (TYPE == kQ6_K)
+            fetch_staged_q6<kHalves>(raw_win + buf * kRawStage, rr,
+                                     210 * (sb0 + sbl) - q6_window_start(sb0 + sbl, (int)p.row_bytes), j, h0, cur);
+          else  // the block of row r sits at r * block bytes: the global fetch code reads it as it is
+            fetch_raw_from<TYPE>(raw_win + buf * kRawStage + rr * Sb<TYPE>::bytes, j, h0, cur[0]);
+#pragma unroll
+          for (int i = 0; i < kHalves; i++) raws[u][i] = cur[i];
+        }
+        if (((ks + kBatch) & 3) == 0) {  // this warp has read all it needs of the window
           __syncwarp();
           if (lane == 0) mbar_arrive(smem_u32(&raw_bars[2 + buf]));
         }
-        mbar_wait(smem_u32(&bars[kEmptyA + s]), ((ks / kStages) & 1) ^ 1);
 #pragma unroll
-        for (int i = 0; i < kHalves; i++)
-          expand_kstep<TYPE, kQuarter>(cur[i], ks0 + ks, h0 + i, smem + s * kStageBytes, r, valid, q2);
+        for (int u = 0; u < kBatch; u++)
+          mbar_wait(smem_u32(&bars[kEmptyA + (ks + u) % kStages]), (((ks + u) / kStages) & 1) ^ 1);
+#pragma unroll
+        for (int u = 0; u < kBatch; u++)
+#pragma unroll
+          for (int i = 0; i < kHalves; i++)
+            expand_kstep<TYPE, kQuarter>(raws[u][i], ks0 + ks + u, h0 + i, smem + ((ks + u) % kStages) * kStageBytes, r, valid, q2);
         fence_async_smem();                                   // generic-proxy writes -> tensor core
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&bars[s]));
+        if (lane < kBatch) mbar_arrive(smem_u32(&bars[(ks + lane) % kStages]));
       }
     } else {
       fetch_all(0, cur);
@@ -906,73 +916,88 @@ __global__ void __launch_bounds__(threads_for(TYPE, STAGED, BN), 1)
     }
   }
   // ---------------------------------------------------------------- epilogue
+  const int q = warp & 3;                                  // TMEM lane quarter this warp may read
+  const uint32_t taddr = tmem_base + ((uint32_t)(32 * q) << 16);
+  // the warps of a lane quarter take an equal share of the token columns each
+  constexpr int kChunks = isolate_mma_warp(TYPE, STAGED, BN) ? 4 : kDequantWarps / 4;
   if (R::in_epilogue(warp)) {
     mbar_wait(smem_u32(&bars[kAccBar]), 0);
     tc_fence_after();
-    const int q = warp & 3;                                // TMEM lane quarter this warp may read
-    const int n = n0 + 32 * q + lane;
-    const uint32_t taddr = tmem_base + ((uint32_t)(32 * q) << 16);
-    // the warps of a lane quarter take an equal share of the token columns each
-    constexpr int kCols = BN / (isolate_mma_warp(TYPE, STAGED, BN) ? 4 : kDequantWarps / 4);
-    const int cbeg = R::epilogue_chunk(warp) * kCols;
-    if constexpr ((kCols / 4) % 32 == 0) {
-      if (p.turns) {  // four splits: the groups of this warp's columns in the order of the turns
-        constexpr int kEpiThreads = 32 * (isolate_mma_warp(TYPE, STAGED, BN) ? 16 : kDequantWarps);
-        constexpr int kG = kCols / 4;
-        unsigned *turn = p.turns + (size_t)(blockIdx.y * gridDim.x + blockIdx.x) * 4;
-        const bool leader = threadIdx.x == (isolate_mma_warp(TYPE, STAGED, BN) ? 0 : 64);
+  }
+  if (p.splits == 1) {
+    if (R::in_epilogue(warp)) {
+      const int n = n0 + 32 * q + lane;
+      constexpr int kCols = BN / kChunks;
+      const int cbeg = R::epilogue_chunk(warp) * kCols;
 #pragma unroll 1
-        for (int t = 0; t < 4; t++) {
-          const int g = ((int)blockIdx.z + t) & 3;
-          if (leader) wait_turn(turn + g, (unsigned)t);
-          asm volatile("bar.sync 2, %0;" ::"n"(kEpiThreads) : "memory");
-#pragma unroll 1
-          for (int c0 = cbeg + g * kG; c0 < cbeg + (g + 1) * kG; c0 += 32) {
-            uint32_t v[32];
-            tmem_ld32(taddr + c0, v);
-            tmem_ld_wait();
-            if (n < p.n_out) {
+      for (int c0 = cbeg; c0 < cbeg + kCols; c0 += 32) {
+        uint32_t v[32];
+        tmem_ld32(taddr + c0, v);
+        tmem_ld_wait();
+        if (n < p.n_out) {
 #pragma unroll
-              for (int jj = 0; jj < 32; jj++) {
-                const int m = m0 + c0 + jj;
-                if (m < p.m_rows) {
-                  float *dst = reinterpret_cast<float *>(p.y) + (long long)m * p.n_out + n;
-                  if (t == 0) *dst = __uint_as_float(v[jj]);  // the group's first part: y needs no zeroing
-                  else atomicAdd(dst, __uint_as_float(v[jj]));
-                }
-              }
+          for (int jj = 0; jj < 32; jj++) {
+            const int m = m0 + c0 + jj;
+            if (m < p.m_rows) {
+              const float f = __uint_as_float(v[jj]);
+              if (p.out_bf16)
+                reinterpret_cast<__nv_bfloat16 *>(p.y)[(long long)m * p.n_out + n] = __float2bfloat16_rn(f);
+              else
+                reinterpret_cast<float *>(p.y)[(long long)m * p.n_out + n] = f;
             }
           }
-          // the additions of all threads happen before the leader's release below (barrier, then a
-          // cumulative gpu-scope release), and the next split's after its leader's acquire
-          asm volatile("bar.sync 2, %0;" ::"n"(kEpiThreads) : "memory");
-          if (leader)
-            asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(turn + g), "r"(t == 3 ? 0u : (unsigned)(t + 1))
-                         : "memory");
         }
       }
     }
-    const bool plain_epilogue = !((kCols / 4) % 32 == 0 && p.turns);
+  } else {
+    // partial tiles: [token column of the round][128 weight rows] f32, at most 128 KB a round
+    constexpr int kRound = BN < 256 ? BN : 256, kCols = kRound / kChunks;
+    static_assert(kRound * kBM * 4 <= kStages * kStageBytes, "a round's partial tile fits the ring");
+    float *part = reinterpret_cast<float *>(smem);
+    const int nw = (int)blockDim.x >> 5, rank = blockIdx.z;
+    const bool vec = (p.n_out & 3) == 0;
 #pragma unroll 1
-    for (int c0 = cbeg; plain_epilogue && c0 < cbeg + kCols; c0 += 32) {
-      uint32_t v[32];
-      tmem_ld32(taddr + c0, v);
-      tmem_ld_wait();
-      if (n < p.n_out) {
+    for (int r0 = 0; r0 < BN && m0 + r0 < p.m_rows; r0 += kRound) {
+      const int live = min(kRound, p.m_rows - m0 - r0);  // columns that are tokens
+      if (R::in_epilogue(warp)) {
+        const int cbeg = R::epilogue_chunk(warp) * kCols;
+#pragma unroll 1
+        for (int c0 = cbeg; c0 < cbeg + kCols && c0 < live; c0 += 32) {
+          uint32_t v[32];
+          tmem_ld32(taddr + r0 + c0, v);
+          tmem_ld_wait();
 #pragma unroll
-        for (int jj = 0; jj < 32; jj++) {
-          const int m = m0 + c0 + jj;
-          if (m < p.m_rows) {
-            const float f = __uint_as_float(v[jj]);
-            if (p.splits > 1)  // two partial tiles onto zeros: the sum does not depend on their order
-              atomicAdd(reinterpret_cast<float *>(p.y) + (long long)m * p.n_out + n, f);
-            else if (p.out_bf16)
-              reinterpret_cast<__nv_bfloat16 *>(p.y)[(long long)m * p.n_out + n] = __float2bfloat16_rn(f);
-            else
-              reinterpret_cast<float *>(p.y)[(long long)m * p.n_out + n] = f;
-          }
+          for (int jj = 0; jj < 32; jj++) part[(c0 + jj) * kBM + 32 * q + lane] = __uint_as_float(v[jj]);
         }
       }
+      split_sync();
+      // a warp takes whole columns: four weight rows a lane, 512 contiguous bytes of every part
+      const int n = n0 + 4 * lane;
+      for (int c = rank + p.splits * warp; c < live; c += p.splits * nw) {
+        const uint32_t own = smem_u32(part + c * kBM + 4 * lane);
+        float4 a = ld_peer4(peer_smem(own, 0));
+        for (int z = 1; z < p.splits; z++) {
+          const float4 b = ld_peer4(peer_smem(own, z));
+          a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+        }
+        const long long at = (long long)(m0 + r0 + c) * p.n_out + n;
+        if (vec && n < p.n_out) {
+          if (p.out_bf16)
+            *reinterpret_cast<uint2 *>(reinterpret_cast<__nv_bfloat16 *>(p.y) + at) =
+                make_uint2(pack_bf16(a.x, a.y), pack_bf16(a.z, a.w));
+          else
+            *reinterpret_cast<float4 *>(reinterpret_cast<float *>(p.y) + at) = a;
+        } else {
+          const float f[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+          for (int i = 0; i < 4; i++)
+            if (n + i < p.n_out) {
+              if (p.out_bf16) reinterpret_cast<__nv_bfloat16 *>(p.y)[at + i] = __float2bfloat16_rn(f[i]);
+              else reinterpret_cast<float *>(p.y)[at + i] = f[i];
+            }
+        }
+      }
+      split_sync();  // the parts are overwritten by the next round, or the CTA leaves
     }
   }
 
@@ -1278,36 +1303,66 @@ EncodeTiledFn encode_tiled_fn() {
   return fn;
 }
 
-// The turn counters of the ordered four-way split: one region of the static device array per
-// (device, stream) that has used it, so that launches on different streams do not share counters.
-constexpr int kTurnSlots = 8, kTurnTiles = 64;
-std::mutex g_turn_mutex;
-unsigned *g_turn_base[64] = {nullptr};
-cudaStream_t g_turn_streams[64][kTurnSlots];
-int g_turn_nstreams[64] = {0};
-unsigned *turn_region(cudaStream_t s) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  std::lock_guard<std::mutex> lock(g_turn_mutex);
-  if (!g_turn_base[dev]) {
-    void *a = nullptr;
-    if (cudaGetSymbolAddress(&a, g_prefill_turns) != cudaSuccess || !a) return nullptr;
-    g_turn_base[dev] = static_cast<unsigned *>(a);
-  }
-  int slot = -1;
-  for (int i = 0; i < g_turn_nstreams[dev]; i++)
-    if (g_turn_streams[dev][i] == s) slot = i;
-  if (slot < 0) {
-    if (g_turn_nstreams[dev] == kTurnSlots) return nullptr;
-    slot = g_turn_nstreams[dev]++;
-    g_turn_streams[dev][slot] = s;
-  }
-  return g_turn_base[dev] + (size_t)slot * kTurnTiles * 4;
-}
-
 int g_prefill_force_bn = 0;  // diagnostics: 0 = automatic, else the token-tile width to use
 int g_prefill_stage_raw = 1;    // diagnostics: 0 = dequant threads read global memory directly
-int g_prefill_force_split = 0;  // diagnostics: 0 = automatic, 1 = never split along K, 2 = two splits where allowed, 3 = four
+int g_prefill_force_split = 0;  // diagnostics: 0 = automatic, 1 = never split along K, 2 / 3 / 4 = two / four / eight splits where allowed
+
+// k-steps of a part of an n-way split: whole superblocks
+int ksteps_per_split(int nks, int splits) { return splits > 1 ? ((nks + splits - 1) / splits + 3) / 4 * 4 : nks; }
+
+template <int TYPE, int BN, bool STAGED>
+constexpr int smem_for() {
+  return stages_for(BN, raw_bytes(TYPE, STAGED)) * (kATile + BN * kBK * 2) + raw_bytes(TYPE, STAGED) +
+         1024 /*alignment*/ + 256 /*barriers*/;
+}
+template <int TYPE, int BN, bool STAGED>
+int configure(int dev) {  // opts into the shared memory, once per device
+  static bool configured[64] = {false};
+  if (dev < 0 || dev >= 64 || configured[dev]) return COGNI_QMM_OK;
+  cudaError_t e = cudaFuncSetAttribute(gemm_prefill_kernel<TYPE, BN, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       smem_for<TYPE, BN, STAGED>());
+  if (e != cudaSuccess) return (int)e;
+  configured[dev] = true;
+  return COGNI_QMM_OK;
+}
+void split_launch_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr, dim3 grid, int threads, int smem,
+                         int splits, cudaStream_t s) {
+  cfg = cudaLaunchConfig_t{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 1;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = splits;
+  cfg.attrs = &attr;
+  cfg.numAttrs = splits > 1 ? 1 : 0;
+}
+
+// How many clusters of `splits` CTAs run at once (every instance takes a whole SM's shared memory,
+// so the narrowest one stands for all).
+int split_capacity(int dev, int splits) {
+  static std::atomic<int> cached[64][4];  // for 2, 4, 8 CTAs: 1 + the count
+  if (dev < 0 || dev >= 64) return 0;
+  std::atomic<int> &slot = cached[dev][splits == 2 ? 1 : splits == 4 ? 2 : 3];
+  int v = slot.load();
+  if (v == 0) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    split_launch_config(cfg, attr, dim3(1, 1, splits), threads_for(kQ4_K, true, 128), smem_for<kQ4_K, 128, true>(),
+                        splits, nullptr);
+    int n = 0;
+    if (configure<kQ4_K, 128, true>(dev) != COGNI_QMM_OK ||
+        cudaOccupancyMaxActiveClusters(&n, gemm_prefill_kernel<kQ4_K, 128, true>, &cfg) != cudaSuccess || n < 0) {
+      cudaGetLastError();  // no split then
+      n = 0;
+    }
+    v = n + 1;
+    slot.store(v);
+  }
+  return v - 1;
+}
 
 template <int TYPE, int BN, bool STAGED>
 int launch(const void *d_w, const void *d_x, void *d_y, int out_type, int m_rows, int n_out,
@@ -1336,17 +1391,10 @@ int launch(const void *d_w, const void *d_x, void *d_y, int out_type, int m_rows
                        strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (cr != CUDA_SUCCESS) return (int)cr;
-  constexpr int smem = stages_for(BN, raw_bytes(TYPE, STAGED)) * (kATile + BN * kBK * 2) +
-                       raw_bytes(TYPE, STAGED) + 1024 /*alignment*/ + 256 /*barriers*/;
-  static bool configured[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && !configured[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_prefill_kernel<TYPE, BN, STAGED>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    configured[dev] = true;
-  }
+  const int st = configure<TYPE, BN, STAGED>(dev);
+  if (st) return st;
   GemmParams p;
   p.w = static_cast<const uint8_t *>(d_w);
   p.y = d_y;
@@ -1356,19 +1404,12 @@ int launch(const void *d_w, const void *d_x, void *d_y, int out_type, int m_rows
   if (!STAGED) tmap_w = tmap;  // unused by the kernel
   const int nks = k_in / kBK;
   p.splits = splits;
-  p.ks_per_split = splits > 1 ? ((nks + splits - 1) / splits + 3) / 4 * 4 : nks;  // whole superblocks
-  p.turns = nullptr;
-  if (splits == 4) {  // the caller has checked that the tiles fit the region and the SMs
-    p.turns = turn_region(s);
-    if (!p.turns) return COGNI_QMM_ERR_LIMIT;
-  }
-  if (splits == 2) {  // (four ordered splits store their first part)
-    cudaError_t e = cudaMemsetAsync(d_y, 0, (size_t)m_rows * n_out * sizeof(float), s);
-    if (e != cudaSuccess) return (int)e;
-  }
-  dim3 grid((n_out + kBM - 1) / kBM, (m_rows + BN - 1) / BN, splits);
-  gemm_prefill_kernel<TYPE, BN, STAGED><<<grid, threads_for(TYPE, STAGED, BN), smem, s>>>(tmap, tmap_w, p);
-  return (int)cudaGetLastError();
+  p.ks_per_split = ksteps_per_split(nks, splits);
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr;
+  split_launch_config(cfg, attr, dim3((n_out + kBM - 1) / kBM, (m_rows + BN - 1) / BN, splits),
+                      threads_for(TYPE, STAGED, BN), smem_for<TYPE, BN, STAGED>(), splits, s);
+  return (int)cudaLaunchKernelEx(&cfg, gemm_prefill_kernel<TYPE, BN, STAGED>, tmap, tmap_w, p);
 }
 
 int g_prefill_pair = 1;  // diagnostics: 0 = the one-CTA kernel for 512-token tiles too
@@ -1419,7 +1460,6 @@ int launch_pair(const void *d_w, const void *d_x, void *d_y, int out_type, int m
   p.row_bytes = row_bytes;
   p.splits = 1;
   p.ks_per_split = k_in / kBK;
-  p.turns = nullptr;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * ((n_out + 2 * kBM - 1) / (2 * kBM)), (m_rows + kPairBN - 1) / kPairBN, 1);
   cfg.blockDim = dim3(kPairThreads);
@@ -1438,11 +1478,14 @@ int launch_pair(const void *d_w, const void *d_x, void *d_y, int out_type, int m
 template <int TYPE>
 int launch_typed(const void *d_w, const void *d_x, void *d_y, int out_type, int m_rows, int n_out,
                  int k_in, cudaStream_t s) {
-  // Token-tile width: wider tiles do less dequant work per flop, narrower ones fill the SMs in
-  // fewer, fuller waves.  Measured time of a tile of 128 / 256 / 512 tokens (in_dim 4096, one wave,
-  // us): Q4_K 39 / 45 / 61 (the 512-token tile on a CTA pair; 63 on one CTA), Q5_K 40 / 45 / 60,
-  // IQ4_NL 49 / 52 / 66, Q6_K 53 / 59 / 69, Q8_0 58 / 67 / 81.  Pick the width with the least
-  // waves x tile time.
+  // Token-tile width and split along K: wider tiles do less dequant work per flop, narrower ones and
+  // splits fill the SMs.  A wave of tiles of 128 / 256 / 512 tokens takes fixed + step x k-steps
+  // (us, fitted to measured launches of one wave with 16 to 192 k-steps; Q6_K rows that TMA cannot
+  // describe are read by the dequant threads and take twice as long), a split adds the exchange of
+  // the partial tiles.  The plan with the least waves x time is taken.  Measured against the whole-K
+  // plans it replaces (us): Q5_K 77 x 4096 x 4096 (m, n, k) 28.3 -> 14.7 (128 tokens, four parts),
+  // Q4_K 20 x 1024 x 4096 19.8 -> 9.2 (eight), Q4_K 300 x 4096 x 4096 32 -> 24.6 (two), Q6_K
+  // 512 x 4096 x 12288 62 -> 55 (four, 512 tokens: atomic turn-taking through global memory before).
   static int sms_of[64] = {0};  // per device: a process may drive GPUs of different sizes
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1453,51 +1496,40 @@ int launch_typed(const void *d_w, const void *d_x, void *d_y, int out_type, int 
     if (dev >= 0 && dev < 64) sms_of[dev] = sms;
   }
   const long long row_tiles = (n_out + kBM - 1) / kBM;
-  const double rel256 = TYPE == kQ4_K || TYPE == kQ5_K || TYPE == kQ8_0 ? 1.15 : 1.10;
-  const double rel512 = TYPE == kQ4_K || TYPE == kQ5_K ? 1.55 : TYPE == kIQ4_NL ? 1.37 : TYPE == kQ8_0 ? 1.41 : 1.31;
-  // Few row tiles against many SMs (a down projection at a short prompt): two CTAs per tile take
-  // half of K each and add their partial tiles onto a zeroed f32 y.  Two addends commute, so the
-  // result stays independent of the order; more splits would not.  The price is the memset of y
-  // and read-modify-write instead of plain stores: about 12 bytes of HBM traffic per output
-  // element, weighed here against the measured time of a 128-token tile's k-step (microseconds).
-  const bool may_split = out_type == COGNI_QMM_OUT_F32 && k_in / kBK >= 16 && g_prefill_force_split != 1;
-  const double us_per_kstep = TYPE == kQ4_K || TYPE == kQ5_K ? 0.61 : TYPE == kIQ4_NL ? 0.76 : TYPE == kQ6_K ? 0.83 : 0.92;
-  const double tile_us = us_per_kstep * (k_in / kBK);
-  const double split_us = 12.0 * (double)m_rows * (double)n_out / 6.0e6;
-  auto cost = [&](int bn, double rel, int splits) {
-    const long long tiles = row_tiles * ((m_rows + bn - 1) / bn) * splits;
-    return (double)((tiles + sms - 1) / sms) * rel * tile_us / splits + (splits > 1 ? split_us : 0.0);
-  };
-  const int widths[3] = {128, 256, 512};
-  const double rels[3] = {1.0, rel256, rel512};
-  int bn = 0, splits = 1;
-  double best = 1e30;
-  for (int i = 0; i < 3; i++) {
-    if (g_prefill_force_bn && g_prefill_force_bn != widths[i]) continue;
-    for (int sp = 1; sp <= (may_split ? 2 : 1); sp++) {
-      if (g_prefill_force_split >= 2 && may_split && sp != 2) continue;
-      const double c = cost(widths[i], rels[i], sp);
-      if (c <= best) { best = c; bn = widths[i]; splits = sp; }
-    }
-  }
-  // Four splits in a fixed order of addition (see wait_turn): 512-token tiles only (the groups of
-  // the epilogue), all CTAs resident at once, a quarter of K of at least 16 k-steps each; costs
-  // the two-split price plus four rounds of turn-taking (about 3 us).
-  {
-    const long long tiles4 = row_tiles * ((m_rows + 511) / 512);
-    const bool can4 = may_split && k_in / kBK >= 64 && tiles4 * 4 <= sms && tiles4 <= kTurnTiles &&
-                      (!g_prefill_force_bn || g_prefill_force_bn == 512);
-    if (can4 && g_prefill_force_split != 2) {
-      const double c4 = rel512 * tile_us / 4 + split_us + 3.0;
-      if (c4 < best || g_prefill_force_split == 3) { best = c4; bn = 512; splits = 4; }
-    }
-  }
+  const long long row_bytes = (long long)(k_in / 256) * Sb<TYPE>::bytes;
   // Rows that are multiples of 16 bytes (always for Q4_K / Q5_K; Q6_K: in_dim a multiple of 2048)
   // of a matrix with at least one full row tile can be fetched by TMA: the raw superblocks of the
   // tile's rows are then staged through shared memory
-  {
-    const long long row_bytes = (long long)(k_in / 256) * Sb<TYPE>::bytes;
-    if (TYPE != kQ8_0 && row_bytes % 16 == 0 && n_out >= kBM && g_prefill_stage_raw) {
+  const bool staged = TYPE != kQ8_0 && row_bytes % 16 == 0 && n_out >= kBM && g_prefill_stage_raw;
+  struct TileTime { double fixed[3], step[3]; };
+  const TileTime tt = TYPE == kQ6_K ? (staged ? TileTime{{6.5, 10.0, 13.0}, {0.62, 0.62, 0.72}}
+                                              : TileTime{{4.0, 8.0, 13.0}, {1.15, 1.30, 1.30}})
+                      : TYPE == kQ8_0   ? TileTime{{5.5, 10.0, 17.5}, {0.76, 0.76, 0.72}}
+                      : TYPE == kIQ4_NL ? TileTime{{6.8, 10.3, 17.8}, {0.59, 0.56, 0.62}}
+                                        : TileTime{{6.5, 7.5, 14.0}, {0.45, 0.50, 0.65}};
+  // Few row tiles against many SMs (short prompts, narrow matrices): the CTAs of a cluster take
+  // equal parts of K of a tile, at least two superblocks each, none empty.
+  const int nks = k_in / kBK;
+  const int widths[3] = {128, 256, 512};
+  int bn = 0, splits = 0;
+  double best = 1e30;
+  for (int i = 0; i < 3; i++) {
+    if (g_prefill_force_bn && g_prefill_force_bn != widths[i]) continue;
+    for (int sp = 1; sp <= 8; sp *= 2) {
+      const int per = ksteps_per_split(nks, sp);
+      if (sp > 1 && (per < 8 || (sp - 1) * per >= nks || g_prefill_force_split == 1)) continue;
+      const int at_once = sp == 1 ? sms : split_capacity(dev, sp);
+      if (at_once == 0) continue;
+      const long long tiles = row_tiles * ((m_rows + widths[i] - 1) / widths[i]);
+      double t = tt.fixed[i] + tt.step[i] * per;
+      if (sp > 1) t += 1.0 + 0.01 * (m_rows < widths[i] ? m_rows : widths[i]);
+      double c = (double)((tiles + at_once - 1) / at_once) * t;
+      if (g_prefill_force_split >= 2 && sp == 1 << (g_prefill_force_split - 1)) c -= 1e6;
+      if (c < best) { best = c; bn = widths[i]; splits = sp; }
+    }
+  }
+  if constexpr (TYPE != kQ8_0) {
+    if (staged) {
       if constexpr (TYPE == kQ4_K || TYPE == kQ5_K) {
         if (bn == 512 && splits == 1 && g_prefill_pair)
           return launch_pair<TYPE>(d_w, d_x, d_y, out_type, m_rows, n_out, k_in, s);
@@ -1539,12 +1571,7 @@ unsigned gemm_prefill_timeouts() {
 
 int gemm_prefill_reset_timeouts() {
   const unsigned zero = 0;
-  cudaError_t e = cudaMemcpyToSymbol(g_pipe_wait_timeouts, &zero, sizeof(zero));
-  if (e != cudaSuccess) return (int)e;
-  void *turns = nullptr;  // an expired wait can leave turn counters of the ordered split non-zero
-  e = cudaGetSymbolAddress(&turns, g_prefill_turns);
-  if (e != cudaSuccess) return (int)e;
-  return (int)cudaMemset(turns, 0, sizeof(unsigned) * 8 * 64 * 4);
+  return (int)cudaMemcpyToSymbol(g_pipe_wait_timeouts, &zero, sizeof(zero));
 }
 
 }  // namespace cogni

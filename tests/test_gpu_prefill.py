@@ -193,6 +193,26 @@ def test_gemm_four_ordered_splits(cuda, oracle, engine, qtype, m, n, k):
     assert lib.cogni_qmm_wait_timeouts() == 0
 
 
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("split", [54, 59, 69])
+@pytest.mark.parametrize("qtype,m,n,k", [(Q4_K, 17, 130, 4096), (Q5_K, 129, 257, 4352), (Q6_K, 257, 150, 4096),
+                                         (Q6_K, 1, 37, 4352), (Q8_0, 600, 129, 4096), (IQ4_NL, 128, 512, 4096)])
+def test_gemm_cluster_splits(cuda, oracle, engine, qtype, m, n, k, split, out_dtype):
+    """Two, four and eight CTAs of a cluster per tile, their partial tiles summed through distributed
+    shared memory: ragged tokens and rows (n not a multiple of 4 takes the scalar stores), unequal
+    parts, both output types.  f32: the additions' order only, 1e-4; bf16 on top: half a unit in the
+    last place of a result of eight significant bits, at most 2^-8 of it (762.1 -> 764 is 2^-8.6)."""
+    engine.lib.cogni_qmm_set_kernel_choice(split)
+    try:
+        w, x, y, ref = run_case(cuda, oracle, qtype, m, n, k, seed=19, out_dtype=out_dtype)
+    finally:
+        engine.lib.cogni_qmm_set_kernel_choice(52)
+    tol = 1e-4 if out_dtype == torch.float32 else 1e-4 + 2.0 ** -8
+    assert not np.isnan(y).any()
+    assert np.abs(y - ref).max() <= tol * np.abs(ref).max()
+    assert engine.lib.cogni_qmm_wait_timeouts() == 0
+
+
 @pytest.mark.parametrize("qtype,n,k", [(Q4_K, 1024, 4096), (Q6_K, 512, 12288), (Q8_0, 512, 4096),
                                        (IQ4_NL, 256, 2048)])
 def test_gemm_within_stated_tolerance_of_cpu_quant_matmul(cuda, oracle, qtype, n, k):
