@@ -1,0 +1,62 @@
+"""Kernels that work block by block: the f32 GEMV of Q8_0 / IQ4_NL rows of any width and the
+dequantiser's 16-byte stores, at the edges of their tiles, and their general forms for unaligned
+buffers.
+
+The GEMV computes d * q (exact quants, one rounding) and accumulates in f32: a lane adds at most 2
+products in sequence per 256 columns and warp, the rest is a tree, so its error against the f64 oracle
+stays below in_dim / 256 + 16 roundings of 2^-24 on the sum of the magnitudes; 1e-5 of max|y| has a
+wide margin at these widths (measured 2e-7)."""
+import numpy as np
+import pytest
+import torch
+
+from cogni_ml_b200 import DeviceQuantWeight, QuantWeight, synth
+
+pytestmark = pytest.mark.gpu
+Q8_0, Q4_K, Q5_K, Q6_K, IQ4_NL = synth.Q8_0, synth.Q4_K, synth.Q5_K, synth.Q6_K, synth.IQ4_NL
+
+
+def aligned_at(host: np.ndarray, offset: int, cuda) -> torch.Tensor:
+    """`host` on the device, `offset` bytes past a 16-byte boundary."""
+    raw = torch.from_numpy(np.ascontiguousarray(host).view(np.uint8).reshape(-1))
+    buf = torch.empty(raw.numel() + 32, dtype=torch.uint8, device=cuda)
+    start = (-buf.data_ptr()) % 16 + offset
+    view = buf[start:start + raw.numel()]
+    view.copy_(raw)
+    return view
+
+
+@pytest.mark.parametrize("qtype", [Q8_0, IQ4_NL])
+@pytest.mark.parametrize("batch", [1, 2, 3, 4, 5, 6, 7, 9, 16, 19])
+@pytest.mark.parametrize("out_dim,in_dim", [(1, 32), (37, 288), (1185, 2080), (2053, 2976), (4738, 544)])
+def test_gemv_of_whole_blocks(cuda, oracle, qtype, batch, out_dim, in_dim):
+    w = synth.make_weight(qtype, out_dim, in_dim, seed=41, tensor_id=qtype)
+    x = synth.make_activation(batch, in_dim, seed=41)
+    res = synth.make_activation(batch, out_dim, 41, 5)
+    dw = DeviceQuantWeight.upload(QuantWeight(w, qtype, out_dim, in_dim), cuda)
+    zero = np.zeros(out_dim, np.float32)
+    ref = oracle.matmul_add(x, batch, in_dim, w, qtype, out_dim, zero, threads=oracle.max_threads()).reshape(batch, out_dim)
+    y = torch.full((batch, out_dim), float("nan"), device=cuda)
+    dw.gemv(torch.from_numpy(x).to(cuda), out=y, residual=torch.from_numpy(res).to(cuda))
+    assert np.abs(y.cpu().numpy() - (ref + res)).max() <= 1e-5 * np.abs(ref).max()
+    # activations on a 4-byte boundary take the row-per-warp kernel
+    xo = aligned_at(x, 4, cuda).view(torch.float32).view(batch, in_dim)
+    assert np.abs(dw.gemv(xo).cpu().numpy() - ref).max() <= 1e-5 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("qtype", [Q8_0, Q4_K, Q5_K, Q6_K, IQ4_NL])
+@pytest.mark.parametrize("blocks", [1, 7, 33, 129])
+@pytest.mark.parametrize("w_at,y_at", [(0, 0), (2, 0), (0, 4)])
+def test_dequantize_tiles_and_alignment(cuda, oracle, engine, qtype, blocks, w_at, y_at):
+    be = 32 if qtype in (Q8_0, IQ4_NL) else 256
+    n = blocks * be
+    w = synth.make_weight(qtype, 1, n, seed=43, tensor_id=qtype)
+    raw = aligned_at(w, w_at, cuda)
+    buf = torch.full((n + 8,), 7.0, device=cuda)
+    start = (-buf.data_ptr()) % 16 // 4 + y_at // 4
+    out = buf[start:start + n]
+    st = engine.lib.cogni_qmm_dequantize(qtype, raw.data_ptr(), n, out.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert st == 0
+    ref = oracle.dequantize(qtype, w, n)
+    assert np.array_equal(out.cpu().numpy().view(np.uint32), ref.view(np.uint32))
+    assert buf[:start].eq(7.0).all() and buf[start + n:].eq(7.0).all()
