@@ -3,7 +3,8 @@
 //
 // This kernel accepts every legal shape (any out_dim, any in_dim that is a block multiple,
 // any batch, 2-byte aligned rows) and is the path for shapes the tiled tensor-core GEMV
-// does not take.  It also carries the fused lm_head variant: GEMV + per-part top-1 +
+// does not take (Q8_0 / IQ4_NL with 16-byte aligned activations: the block kernel further down).
+// It also carries the fused lm_head variant: GEMV + per-part top-1 +
 // last-CTA-done reduction, all in one launch.
 //
 // Weight value arithmetic follows src/ml/gguf/quant_matmul.cr (w = d*sc*q - dmin*m for
@@ -162,6 +163,131 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32)
   }
 }
 
+// Q8_0 / IQ4_NL rows of any whole number of 32-element blocks (widths that no 256-element superblock
+// divides; in f32 throughout).  A row of such a matrix is a few kilobytes, so what bounds the
+// row-per-warp kernel above is latency: one block after the other, two bytes a load.  Here a warp
+// takes eight blocks of RPW rows at a time, four lanes per block and eight weights per lane; the
+// activations are read as 16-byte vectors once for the RPW rows, and `wk` of a CTA's eight warps split
+// K (partial sums meet in shared memory and are added in warp order: the same bits every time).  The
+// columns of one row group are neighbouring CTAs, so the weights come from DRAM once.  Measured against
+// the row-per-warp kernel (us): IQ4_NL 2053 x 2976 batch 1 / 3 / 16 14.1 -> 5.5 / 21.9 -> 6.4 / 102 ->
+// 20, Q8_0 100 x 10016 batch 8 148 -> 6.2, Q8_0 20000 x 10016 batch 1 / 8 147 -> 68 (3.1 TB/s) / 855 ->
+// 221 (then bound by its f32 arithmetic, 7 instructions per weight beside the multiply-adds).
+constexpr int kBlockWarps = 8;
+template <int TYPE>
+__device__ __forceinline__ void load_quants(const uint8_t *blk, int p, uint32_t (&q)[2], float &d) {
+  // 2-byte aligned addresses.  Elements 4p .. 4p+3 and 16+4p .. 16+4p+3 of the block.
+  auto word = [](const uint8_t *a) {
+    const unsigned short *h = reinterpret_cast<const unsigned short *>(a);
+    return (uint32_t)__ldg(h) | (uint32_t)__ldg(h + 1) << 16;
+  };
+  d = __half2float(__ushort_as_half(__ldg(reinterpret_cast<const unsigned short *>(blk))));
+  q[0] = word(blk + 2 + 4 * p);
+  q[1] = TYPE == kQ8_0 ? word(blk + 18 + 4 * p) : 0u;
+}
+// the eight weights d * q, elements 4p .. 4p+3, then 16+4p .. 16+4p+3
+template <int TYPE>
+__device__ __forceinline__ void block_weights(const uint32_t (&q)[2], float d, float (&v)[8]) {
+  uint32_t b[2];  // signed bytes
+  if constexpr (TYPE == kQ8_0) {
+    b[0] = q[0];
+    b[1] = q[1];
+  } else {
+    auto lut4 = [](uint32_t h) {  // nibbles 0 .. 3 of h -> the four table values as bytes
+      const uint32_t s7 = h & 0x7777u;
+      const uint32_t lo = __byte_perm(0xBFAD9881u, 0xF6EADDCFu, s7);  // entries 0 .. 7
+      const uint32_t hi = __byte_perm(0x26190D01u, 0x71594535u, s7);  // entries 8 .. 15
+      return __byte_perm(lo, hi, 0x3210u | ((h >> 1) & 0x4444u));
+    };
+    const uint32_t e = lut4(q[0]), o = lut4(q[0] >> 16);  // (low, high) nibble pairs of bytes 0, 1 | 2, 3
+    b[0] = __byte_perm(e, o, 0x6420);
+    b[1] = __byte_perm(e, o, 0x7531);
+  }
+#pragma unroll
+  for (int i = 0; i < 8; i++)  // the float is 2^23 + 128 + b, exactly
+    v[i] = d * (__uint_as_float(__byte_perm(b[i >> 2] ^ 0x80808080u, 0x4B000000u, 0x7650 + (i & 3))) - 8388736.f);
+}
+
+template <int TYPE, int NB, int RPW>
+__global__ void __launch_bounds__(kBlockWarps * 32)
+    gemv_blocks_kernel(const uint8_t *__restrict__ w, const float *__restrict__ x, const float *addend,
+                       int64_t addend_stride, float *y, int in_dim, int out_dim, int batch, int bgroups,
+                       int wk) {
+  constexpr int BB = BlockGeom<TYPE>::bytes;
+  constexpr int NP = NB == 3 ? 4 : NB > 4 ? 8 : NB, N = RPW * NP;  // sums of a warp, columns padded to a power of two
+  __shared__ float s_part[kBlockWarps][N];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, p = lane & 3;
+  const int nblk = in_dim >> 5;
+  const int kw = warp & (wk - 1), grp = warp / wk;  // this warp's part of K, its row group of the CTA
+  const int row0 = ((int)(blockIdx.x / bgroups) * (kBlockWarps / wk) + grp) * RPW;
+  const int b0 = min((int)(blockIdx.x % bgroups) * NB, batch - NB);  // the last group overlaps the one before
+  const long long row_bytes = (long long)nblk * BB;
+  const uint8_t *wr[RPW];
+#pragma unroll
+  for (int r = 0; r < RPW; r++) wr[r] = w + (long long)min(row0 + r, out_dim - 1) * row_bytes;
+  const float *xb = x + (long long)b0 * in_dim + 4 * p;
+  float acc[N];
+#pragma unroll
+  for (int i = 0; i < N; i++) acc[i] = 0.f;
+  for (int blk = 8 * kw + (lane >> 2); blk < nblk; blk += 8 * wk) {
+    uint32_t q[RPW][2];
+    float d[RPW];
+#pragma unroll
+    for (int r = 0; r < RPW; r++) load_quants<TYPE>(wr[r] + (long long)blk * BB, p, q[r], d[r]);
+    float v[RPW][8];
+#pragma unroll
+    for (int r = 0; r < RPW; r++) block_weights<TYPE>(q[r], d[r], v[r]);
+#pragma unroll
+    for (int c = 0; c < NB; c++) {
+      const float4 *xp = reinterpret_cast<const float4 *>(xb + (long long)c * in_dim + 32 * blk);
+      const float4 xl = __ldg(xp), xh = __ldg(xp + 4);
+#pragma unroll
+      for (int r = 0; r < RPW; r++) {
+        float s = fmaf(v[r][0], xl.x, acc[r * NP + c]);
+        s = fmaf(v[r][1], xl.y, s);
+        s = fmaf(v[r][2], xl.z, s);
+        s = fmaf(v[r][3], xl.w, s);
+        s = fmaf(v[r][4], xh.x, s);
+        s = fmaf(v[r][5], xh.y, s);
+        s = fmaf(v[r][6], xh.z, s);
+        acc[r * NP + c] = fmaf(v[r][7], xh.w, s);
+      }
+    }
+  }
+  // sum over the lanes: while there are several sums, half of the lanes keep one half of them
+  int n = N, off = 16;
+#pragma unroll
+  for (int step = 0; step < 5; step++) {
+    if (n > 1) {
+      n >>= 1;
+      const bool up = (lane & off) != 0;
+#pragma unroll
+      for (int i = 0; i < N / 2; i++)
+        if (i < n) {
+          const float keep = up ? acc[i + n] : acc[i], give = up ? acc[i] : acc[i + n];
+          acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+        }
+    } else {
+      acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], off);
+    }
+    off >>= 1;
+  }
+  constexpr int kLanesPerSum = 32 / N;  // sum i sits in lanes i * kLanesPerSum ..
+  if (lane % kLanesPerSum == 0) s_part[warp][lane / kLanesPerSum] = acc[0];
+  __syncthreads();
+  if (threadIdx.x < N * kBlockWarps && threadIdx.x / N < kBlockWarps / wk) {
+    const int g = threadIdx.x / N, i = threadIdx.x % N, r = i / NP, c = i % NP;
+    const int row = ((int)(blockIdx.x / bgroups) * (kBlockWarps / wk) + g) * RPW + r;
+    float sum = 0.f;
+    for (int k = 0; k < wk; k++) sum += s_part[g * wk + k][i];
+    const int b = b0 + c;
+    if (c < NB && row < out_dim) {
+      const float a = addend ? addend[(int64_t)b * addend_stride + row] : 0.f;
+      y[(int64_t)b * out_dim + row] = a + sum;
+    }
+  }
+}
+
 // Fused lm_head: each CTA owns kTop1RowsPerPart consecutive rows of one batch row's logits,
 // keeps the best (value, index) key, stores it in its scratch slot; the CTA that takes the
 // last ticket of a batch row folds all slots and writes the result.
@@ -223,10 +349,53 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32)
   }
 }
 
+// Four rows a warp share the activations' loads; matrices of few rows take one row a warp, so that
+// two CTAs per SM remain.  Short rows are split over fewer warps: a part has at least one step of
+// eight blocks, two where the matrix has rows enough to fill the SMs.
+template <int TYPE, int NB, int RPW>
+int run_blocks_rows(const void *d_w, const float *d_x, const float *d_addend, int64_t addend_stride, float *d_y,
+                    int in_dim, int out_dim, int batch, int bgroups, cudaStream_t s) {
+  const int groups = (out_dim + RPW - 1) / RPW, steps = (in_dim / 32 + 7) / 8;
+  int wk = kBlockWarps;
+  while (wk > 1 && (wk / 2 >= steps ||
+                    (wk >= steps && (long long)groups * bgroups * wk / 2 >= 148LL * 4 * kBlockWarps)))
+    wk /= 2;
+  const int per_cta = kBlockWarps / wk;
+  const unsigned ctas = (unsigned)((groups + per_cta - 1) / per_cta) * (unsigned)bgroups;
+  gemv_blocks_kernel<TYPE, NB, RPW><<<ctas, kBlockWarps * 32, 0, s>>>(
+      static_cast<const uint8_t *>(d_w), d_x, d_addend, addend_stride, d_y, in_dim, out_dim, batch, bgroups, wk);
+  return (int)cudaGetLastError();
+}
+template <int TYPE, int NB>
+int run_blocks(const void *d_w, const float *d_x, const float *d_addend, int64_t addend_stride, float *d_y,
+               int in_dim, int out_dim, int batch, int bgroups, cudaStream_t s) {
+  if (NB > 4 || (long long)((out_dim + 3) / 4) * bgroups >= 2 * 148)
+    return run_blocks_rows<TYPE, NB, 4>(d_w, d_x, d_addend, addend_stride, d_y, in_dim, out_dim, batch, bgroups, s);
+  return run_blocks_rows<TYPE, (NB > 4 ? 4 : NB), (NB > 4 ? 4 : 1)>(d_w, d_x, d_addend, addend_stride, d_y, in_dim, out_dim, batch, bgroups, s);
+}
+
 template <int TYPE>
 int run_gemv(const void *d_w, const float *d_x, const float *d_addend, int64_t addend_stride,
              float *d_y, int in_dim, int out_dim, int batch, cudaStream_t s) {
   const uint8_t *w = static_cast<const uint8_t *>(d_w);
+  if constexpr (TYPE == kQ8_0 || TYPE == kIQ4_NL) {
+    // 16-byte loads of x: rows are whole 128-byte blocks, so its base decides
+    // Up to four columns a CTA; on many rows the unpacked weights serve up to eight (Q8_0: six, its
+    // weights take more registers until they are unpacked; 20000 x 10016 at batch 5 / 8: 166 -> 143 /
+    // 221 -> 259 us with one group of 5 / 8 against 3 + 3 / 4 + 4, IQ4_NL 196 -> 165 / 219 -> 191).
+    const int most = batch > 4 && out_dim >= 4 * 148 * 8 ? (TYPE == kIQ4_NL ? 8 : 6) : 4;
+    const int bg = (batch + most - 1) / most, nb = (batch + bg - 1) / bg;  // 5 rows: 3 + 3, 9: 3 + 3 + 3
+    if ((reinterpret_cast<uintptr_t>(d_x) & 15) == 0 && (long long)out_dim * bg <= 0x7fffffffLL) {
+      if (nb == 1) return run_blocks<TYPE, 1>(d_w, d_x, d_addend, addend_stride, d_y, in_dim, out_dim, batch, bg, s);
+      if (nb == 2) return run_blocks<TYPE, 2>(d_w, d_x, d_addend, addend_stride, d_y, in_dim, out_dim, batch, bg, s);
+      if (nb == 3) return run_blocks<TYPE, 3>(d_w, d_x, d_addend, addend_stride, d_y, in_dim, out_dim, batch, bg, s);
+      if (nb == 4) return run_blocks<TYPE, 4>(d_w, d_x, d_addend, addend_stride, d_y, in_dim, out_dim, batch, bg, s);
+      if (nb == 5) return run_blocks<TYPE, 5>(d_w, d_x, d_addend, addend_stride, d_y, in_dim, out_dim, batch, bg, s);
+      if (nb == 6) return run_blocks<TYPE, 6>(d_w, d_x, d_addend, addend_stride, d_y, in_dim, out_dim, batch, bg, s);
+      if (nb == 7) return run_blocks<TYPE, 7>(d_w, d_x, d_addend, addend_stride, d_y, in_dim, out_dim, batch, bg, s);
+      return run_blocks<TYPE, 8>(d_w, d_x, d_addend, addend_stride, d_y, in_dim, out_dim, batch, bg, s);
+    }
+  }
   dim3 grid((out_dim + kWarpsPerCta - 1) / kWarpsPerCta), block(kWarpsPerCta * 32);
   if (batch >= 4)
     gemv_rowwarp_kernel<TYPE, 4><<<grid, block, 0, s>>>(w, d_x, d_addend, addend_stride, d_y,
