@@ -44,6 +44,7 @@ SIGNATURES = {
     "cogni_qmm_top1_unpack_keys": (_i, [_vp, _i, _vp, _vp, _vp]),
     "cogni_qmm_gemm_bf16": (_i, [_i, _vp, _vp, _vp, _i, _i, _i, _i, _vp]),
     "cogni_qmm_matmul_add_host": (_i, [_vp, _i, _i, _vp, _i64, _i, _i, _vp, _vp]),
+    "cogni_qmm_release_host_workspaces": (_i, []),
     # include/cogni_qmm_diag.h
     "cogni_qmm_set_kernel_choice": (_i, [_i]),
     "cogni_qmm_diag_expire_wait": (_i, [C.c_uint, _vp]),

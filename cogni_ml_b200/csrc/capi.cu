@@ -387,28 +387,30 @@ int cogni_qmm_matmul_add_host(const float *x, int rows, int in_dim, const void *
   if (!x || !w_raw || !y || rows <= 0 || in_dim <= 0 || out_dim <= 0) return COGNI_QMM_ERR_ARG;
   int64_t need = cogni_qmm_tensor_bytes(type, out_dim, in_dim);
   if (need < 0 || w_bytes < need) return COGNI_QMM_ERR_ARG;
-  void *d_w = nullptr;
-  float *d_x = nullptr, *d_b = nullptr, *d_y = nullptr;
-  size_t xb = (size_t)rows * in_dim * 4, yb = (size_t)rows * out_dim * 4;
-  int st = COGNI_QMM_OK;
+  const size_t xb = (size_t)rows * in_dim * 4, yb = (size_t)rows * out_dim * 4, bb = bias ? (size_t)out_dim * 4 : 0;
+  auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
+  HostWorkspace ws;
+  int st = (int)host_workspace_take(al((size_t)need) + al(xb) + al(bb) + al(yb), ws);
+  if (st) return st;
+  uint8_t *d_w = static_cast<uint8_t *>(ws.p);
+  float *d_x = reinterpret_cast<float *>(d_w + al((size_t)need));
+  float *d_b = bias ? d_x + al(xb) / 4 : nullptr;
+  float *d_y = d_x + (al(xb) + al(bb)) / 4;
   auto step = [&](cudaError_t e) {
     if (st == COGNI_QMM_OK && e != cudaSuccess) st = (int)e;
     return st == COGNI_QMM_OK;
   };
-  if (step(cudaMalloc(&d_w, (size_t)need)) && step(cudaMalloc(&d_x, xb)) &&
-      step(cudaMalloc(&d_y, yb)) && (!bias || step(cudaMalloc(&d_b, (size_t)out_dim * 4))) &&
-      step(cudaMemcpy(d_w, w_raw, (size_t)need, cudaMemcpyHostToDevice)) &&
+  if (step(cudaMemcpy(d_w, w_raw, (size_t)need, cudaMemcpyHostToDevice)) &&
       step(cudaMemcpy(d_x, x, xb, cudaMemcpyHostToDevice)) &&
-      (!bias || step(cudaMemcpy(d_b, bias, (size_t)out_dim * 4, cudaMemcpyHostToDevice)))) {
+      (!bias || step(cudaMemcpy(d_b, bias, bb, cudaMemcpyHostToDevice)))) {
     st = cogni_qmm_gemv(type, d_w, d_x, d_b, 0, d_y, in_dim, out_dim, rows, nullptr);
     if (st == COGNI_QMM_OK) step(cudaMemcpy(y, d_y, yb, cudaMemcpyDeviceToHost));
     if (st == COGNI_QMM_OK && cogni_qmm_wait_timeouts() != 0) st = COGNI_QMM_ERR_TIMEOUT;
   }
-  cudaFree(d_w);
-  cudaFree(d_x);
-  cudaFree(d_y);
-  cudaFree(d_b);
+  host_workspace_return(ws, st == COGNI_QMM_OK);
   return st;
 }
+
+int cogni_qmm_release_host_workspaces(void) { return host_workspace_release_idle(); }
 
 }  // extern "C"

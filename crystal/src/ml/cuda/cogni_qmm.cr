@@ -105,6 +105,7 @@ lib LibCogniQMM
   fun cogni_qmm_matmul_add_host(x : Float32*, rows : Int32, in_dim : Int32, w_raw : Void*,
                                 w_bytes : Int64, type : Int32, out_dim : Int32, bias : Float32*,
                                 y : Float32*) : Int32
+  fun cogni_qmm_release_host_workspaces : Int32
   # include/cogni_qmm_diag.h
   fun cogni_qmm_set_kernel_choice(choice : Int32) : Int32
   fun cogni_qmm_diag_expire_wait(limit_us : UInt32, stream : Void*) : Int32

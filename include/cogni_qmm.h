@@ -384,6 +384,13 @@ int cogni_qmm_matmul_add_host(const float *x, int rows, int in_dim, const void *
                               int64_t w_bytes, int type, int out_dim, const float *bias,
                               float *y);
 
+/*
+ * The host-buffer form keeps the device memory of its calls (at most 256 MB of the process, one block
+ * per call in flight) for later calls.  This gives the blocks that no call is using, of the current
+ * context, back to the device.  (No counterpart in the reference.)
+ */
+int cogni_qmm_release_host_workspaces(void);
+
 #ifdef __cplusplus
 }
 #endif
