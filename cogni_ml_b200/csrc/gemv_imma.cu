@@ -266,10 +266,29 @@ __device__ __forceinline__ void imma16_zero(int (&d)[4], uint32_t a0, uint32_t a
       : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
       : "r"(a0), "r"(a1), "r"(b0), "r"(0));
 }
+__device__ __forceinline__ void imma16_s8_zero(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+  asm(
+      "mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5}, {%6}, "
+      "{%7,%7,%7,%7};"
+      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+      : "r"(a0), "r"(a1), "r"(b0), "r"(0));
+}
+// byte I of v, sign-extended
+template <int I>
+__device__ __forceinline__ int sbyte(uint32_t v) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(v), "n"(I | (8 | I) << 4 | (8 | I) << 8 | (8 | I) << 12));
+  return (int)r;
+}
 // scale * (byte i of v), exactly rounded once: 0x4B0000bb is the float 2^23 + b, and
 // fma(2^23 + b, scale, -2^23 * scale) = b * scale (the product 2^23 * scale is exact).
 __device__ __forceinline__ float byte_times(uint32_t v, int i, float scale, float scale_2p23) {
   return fmaf(__uint_as_float(__byte_perm(v, 0x4B000000u, 0x7650 + i)), scale, -scale_2p23);
+}
+
+// The largest of the lanes' values, none of them negative or NaN: such floats order like their bits.
+__device__ __forceinline__ float warp_max_nonneg(float v) {
+  return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(v)));
 }
 
 // Shared-memory layout of the quantised activations, in MMA B-fragment order.  A "unit" is 64
@@ -728,46 +747,128 @@ __device__ __forceinline__ void quantise_superblocks(const float *x, const float
 // With more than two batch rows the MMA columns are (batch row b' of a set of four, plane):
 // column 2b' + plane, one MMA per scale group and set (m16n8k32 for the 32-element groups,
 // m16n8k16 for Q6_K's 16-element groups), no structural zeros.  Lane (g, t) of the result holds
-// the hi and lo sums of batch row 4j + t for weight rows g and g+8 of set j.  The warp's area holds
-// d*sc per (row, group) in group order, without the activation scale, which the lane multiplies in
-// per (group, batch row); the row's corrections follow at index NG + b.
-template <int TYPE> struct Dense {
+// the hi and lo sums of batch row 4j + t for weight rows g and g+8 of set j.
+template <int TYPE, int NB> struct Dense {
+  static constexpr int J = NB / 4;                 // sets of four batch rows
   static constexpr int W = TYPE == kQ6_K ? 4 : 8;  // bytes of a lane's B fragment per (group, set)
-  static constexpr int GB = 32 * W;                // bytes of a (group, set)
+  // Bytes of a group: a lane's fragments of all sets side by side, and 16 bytes on top so that the
+  // quantiser's stores, whose lanes sit in different groups, spread over the banks.
+  static constexpr int GB = 32 * W * J + 16;
 };
-// floats per area row: NG scales + NB corrections, padded so that the 8 rows a warp reads with
-// 16-byte loads fall into distinct banks
-__host__ __device__ constexpr int dense_area_row(int ng, int nb) {
-  return nb <= 4 ? ng + 4 : (ng == 8 ? 20 : 28);
-}
+// floats per area row of Q8_0 / IQ4_NL (d per scale group of a row, without the activation scale),
+// padded so that the 8 rows a warp reads with 8-byte loads fall into distinct banks
+__host__ __device__ constexpr int dense_area_row(int ng) { return ng + 4; }
 
-// Quantises superblock kblk of x for NB batch rows (rows beyond `batch` repeat the last one) into
-// the dense fragment order: byte offset ((group * J + set) * 32 + column * 4 + t) * W.
+// The integer-domain loop of the K-quants takes its offset sums (min or scale x group sum of n) from
+// the tensor cores as well: a group sum |n0 + 128 n1 + 16384 n2| < 2^20 is stored as three byte
+// planes in B-fragment order of m16n8k16 (k = group, column 2t = batch row t, 2t + 1 = 4 + t, which
+// is where a lane needs it), the A operand is a row's mins or scales.
+template <int TYPE> struct GroupSums {
+  static constexpr int LANES = TYPE == kQ6_K ? 32 : 16;  // eight groups fill only lanes t < 2
+  static constexpr int WORDS = 3 * LANES;                // per superblock
+};
+
+// Quantises superblock kblk of x for NB batch rows (those beyond `batch` are left out: their columns
+// hold whatever was there, and no result of theirs is stored) into the dense fragment order: byte
+// offset group * GB + ((column * 4 + t) * J + set) * W, so that a lane
+// fetches its fragments of all sets of a group at once.  Batch rows b and b + 4 (the same column of
+// two sets) are stored together, 16 bytes a lane and plane (one set: 8): 32 lanes write 512 bytes in
+// the four wavefronts that these take; an 8-byte store per row and plane, the groups 512 bytes apart,
+// took eight, and IQ4_NL's single bytes far more.
+// IQ4_NL 1024 x 4096 at batch 8 15.4 -> 7.9 us, 12288 x 4096 at batch 4 19.0 -> 15.4.
 // SB: one scale per superblock and batch row (SX[kblk * NB + b]) and the groups' integer sums of n
-// in XX, for the integer-domain loop of the K-quants; otherwise one scale per group.
+// in XX (GroupSums), for the integer-domain loop of the K-quants; otherwise one scale per group.
 template <int TYPE, int NB, bool LL, bool SB>
 __device__ __forceinline__ void quantise_dense(const float *x, const float *x_up,
                                                const float *norm_w, const float *inv_rms, int K,
                                                int batch, int kblk, int lane, uint8_t *xq,
                                                float *SX, float *XX, const XSrc &src) {
   using C = Cfg<TYPE>;
-  constexpr int J = NB / 4, W = Dense<TYPE>::W;
+  using D = Dense<TYPE, NB>;
+  constexpr int J = D::J, W = D::W;
   constexpr int LPG = C::GROUP / 8;  // lanes per scale group
   const int k = kblk * 256 + lane * 8;
   const int grp = k / C::GROUP;
-  // this lane's 8 bytes inside a column's 4 * W: lanes t of the MMA take W bytes each
-  const int tpos = (lane & (LPG - 1)) * 8;
+  // this lane's 8 quants of a column are the 8 bytes of lane t of the MMA (W = 8), or those of t, t + 1
+  const int c = lane & (LPG - 1);
+  const int t = TYPE == kIQ4_NL ? 2 * (c & 1) + (c >> 1) : W == 8 ? c : 2 * c;
+  uint8_t *dst0 = xq + (size_t)grp * D::GB + t * J * W;
   float4 w0 = make_float4(1.f, 1.f, 1.f, 1.f), w1 = w0;
   if (norm_w) {
     w0 = __ldg(reinterpret_cast<const float4 *>(norm_w + k));
     w1 = __ldg(reinterpret_cast<const float4 *>(norm_w + k + 4));
   }
+  // the quants of batch row b as two words per plane, in the order of the fragments
+  auto quantise_row = [&](int b, const float4 &a0, const float4 &a1, uint32_t (&hw)[2], uint32_t (&lw)[2]) {
+    const float v[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+    float mx = 0.f;
 #pragma unroll
-  for (int b4 = 0; b4 < NB; b4 += 4) {
+    for (int e = 0; e < 8; e++) mx = fmaxf(mx, fabsf(v[e]));
+    if constexpr (SB) {
+      mx = warp_max_nonneg(mx);
+    } else {
+#pragma unroll
+      for (int off = 1; off < LPG; off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+    }
+    const bool live = mx > 1e-30f;  // as in quantise_superblocks
+    const float sx = live ? mx * (1.f / kNMax) : 1.f;
+    const float inv = live ? (float)kNMax / mx : 0.f;
+    uint32_t bits[8], up[8];
+    int nsum = 0;
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+      bits[e] = __float_as_uint(fmaf(v[e], inv, 12582912.f));
+      up[e] = bits[e] << 1;
+      nsum += (int)(bits[e] - 0x4B400000u);
+    }
+    if constexpr (SB) {
+#pragma unroll
+      for (int off = 1; off < LPG; off <<= 1) nsum += __shfl_xor_sync(0xffffffffu, nsum, off);
+      if (lane == 0) SX[kblk * NB + b] = sx;
+      if (c == 0) {
+        constexpr int L = GroupSums<TYPE>::LANES;
+        const int gi = grp & (C::NG - 1), col = b < 4 ? 2 * b : 2 * b - 7;
+        uint8_t *w = reinterpret_cast<uint8_t *>(XX) +
+                     ((size_t)kblk * GroupSums<TYPE>::WORDS + col * (L / 8) + (gi >> 2)) * 4 + (gi & 3);
+        w[0] = (uint8_t)(nsum & 127);
+        w[4 * L] = (uint8_t)((nsum >> 7) & 127);
+        w[8 * L] = (uint8_t)(nsum >> 14);
+      }
+    } else if (c == 0) {
+      SX[grp * NB + b] = sx;
+    }
+#pragma unroll
+    for (int w4 = 0; w4 < 2; w4++) {
+      lw[w4] = __byte_perm(__byte_perm(bits[4 * w4], bits[4 * w4 + 1], 0x0040),
+                           __byte_perm(bits[4 * w4 + 2], bits[4 * w4 + 3], 0x0040), 0x5410) & 0x7f7f7f7fu;
+      hw[w4] = __byte_perm(__byte_perm(up[4 * w4], up[4 * w4 + 1], 0x0051),
+                           __byte_perm(up[4 * w4 + 2], up[4 * w4 + 3], 0x0051), 0x5410);
+    }
+    if constexpr (TYPE == kIQ4_NL) {
+      // The A fragments come out of the nibble table in the order (element i, element 16 + i,
+      // element i + 1, element 17 + i) per pair of weight bytes, so the activations are laid out to
+      // match: lane c holds elements 8c .. 8c+7, lane c ^ 2 those 16 away; the lower of the two keeps
+      // the first four pairs, the upper one the last four.
+#pragma unroll
+      for (int pl = 0; pl < 2; pl++) {
+        uint32_t(&q)[2] = pl ? lw : hw;
+        const bool low = c < 2;
+        const uint32_t own = low ? q[0] : q[1], other = __shfl_xor_sync(0xffffffffu, low ? q[1] : q[0], 2);
+        const uint32_t first = low ? own : other, second = low ? other : own;
+        q[0] = __byte_perm(first, second, 0x5140);
+        q[1] = __byte_perm(first, second, 0x7362);
+      }
+    }
+  };
+  // four rows' loads at a time, two of each set (J = 1: the four rows)
+#pragma unroll
+  for (int i0 = 0; i0 < 4; i0 += 4 / J) {
     float4 v0[4], v1[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-      const int br = min(b4 + i, batch - 1);
+      const int br = J == 2 ? i0 + (i & 1) + 4 * (i >> 1) : i;
+      v0[i] = v1[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (br >= batch) continue;
       const long long off = (long long)br * K + k;
       v0[i] = ld4x<LL>(x, off, src);
       v1[i] = ld4x<LL>(x, off + 4, src);
@@ -785,135 +886,70 @@ __device__ __forceinline__ void quantise_dense(const float *x, const float *x_up
       }
     }
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int b = b4 + i;
-      const float v[8] = {v0[i].x, v0[i].y, v0[i].z, v0[i].w, v1[i].x, v1[i].y, v1[i].z, v1[i].w};
-      float mx = 0.f;
-#pragma unroll
-      for (int e = 0; e < 8; e++) mx = fmaxf(mx, fabsf(v[e]));
-#pragma unroll
-      for (int off = 1; off < (SB ? 32 : LPG); off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-      const bool live = mx > 1e-30f;  // as in quantise_superblocks
-      const float sx = live ? mx * (1.f / kNMax) : 1.f;
-      const float inv = live ? (float)kNMax / mx : 0.f;
-      uint32_t bits[8], up[8];
-      int nsum = 0;
-#pragma unroll
-      for (int e = 0; e < 8; e++) {
-        bits[e] = __float_as_uint(fmaf(v[e], inv, 12582912.f));
-        up[e] = bits[e] << 1;
-        nsum += (int)(bits[e] - 0x4B400000u);
-      }
-#pragma unroll
-      for (int off = 1; off < LPG; off <<= 1) nsum += __shfl_xor_sync(0xffffffffu, nsum, off);
-      if constexpr (SB) {
-        if (lane == 0) SX[kblk * NB + b] = sx;
-        if ((lane & (LPG - 1)) == 0) reinterpret_cast<int *>(XX)[grp * NB + b] = nsum;
-      } else if ((lane & (LPG - 1)) == 0) {
-        SX[grp * NB + b] = sx;
-        XX[grp * NB + b] = sx * (float)nsum;
-      }
-      uint32_t lw[2], hw[2];
-#pragma unroll
-      for (int w4 = 0; w4 < 2; w4++) {
-        lw[w4] = __byte_perm(__byte_perm(bits[4 * w4], bits[4 * w4 + 1], 0x0040),
-                             __byte_perm(bits[4 * w4 + 2], bits[4 * w4 + 3], 0x0040), 0x5410) & 0x7f7f7f7fu;
-        hw[w4] = __byte_perm(__byte_perm(up[4 * w4], up[4 * w4 + 1], 0x0051),
-                             __byte_perm(up[4 * w4 + 2], up[4 * w4 + 3], 0x0051), 0x5410);
-      }
-      uint8_t *dst = xq + ((size_t)(grp * J + (b >> 2)) * 32 + 2 * (b & 3) * 4) * W + tpos;
-      if constexpr (TYPE == kIQ4_NL) {
-        // The A fragments come out of the nibble table in the order (element i, element 16 + i,
-        // element i + 1, element 17 + i) per pair of weight bytes, so the activations are laid out
-        // to match: element e of the block (byte be = e & 15 of its 16, nibble e >> 4) goes to
-        // MMA lane t = be >> 2, word m = (be >> 1) & 1, byte 2 * (be & 1) + (e >> 4).
-        const int c = lane & 3;  // this lane holds elements 8c .. 8c + 7
-        uint8_t *col = dst - tpos;
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const int off = (2 * (c & 1) + (i >> 2)) * 8 + ((i >> 1) & 1) * 4 + 2 * (i & 1) + (c >> 1);
-          col[off] = (uint8_t)(hw[i >> 2] >> (8 * (i & 3)));
-          col[off + 4 * W] = (uint8_t)(lw[i >> 2] >> (8 * (i & 3)));
-        }
+    for (int i = 0; i < 4 / J; i++) {
+      const int b = i0 + i;
+      uint8_t *dst = dst0 + 2 * b * 4 * J * W;  // hi plane: column 2b; lo plane: column 2b + 1
+      if (b >= batch) break;
+      uint32_t h0[2], l0[2];
+      quantise_row(b, v0[i], v1[i], h0, l0);
+      if constexpr (J == 2) {
+        uint32_t h1[2] = {0u, 0u}, l1[2] = {0u, 0u};
+        if (b + 4 < batch) quantise_row(b + 4, v0[i + 2], v1[i + 2], h1, l1);
+        constexpr bool wide = W == 8;  // a lane's two words of one set, or the two sets of one word, side by side
+        *reinterpret_cast<uint4 *>(dst) = make_uint4(h0[0], wide ? h0[1] : h1[0], wide ? h1[0] : h0[1], h1[1]);
+        *reinterpret_cast<uint4 *>(dst + 4 * J * W) =
+            make_uint4(l0[0], wide ? l0[1] : l1[0], wide ? l1[0] : l0[1], l1[1]);
       } else {
-        *reinterpret_cast<uint2 *>(dst) = make_uint2(hw[0], hw[1]);          // hi plane: column 2b'
-        *reinterpret_cast<uint2 *>(dst + 4 * W) = make_uint2(lw[0], lw[1]);  // lo plane: column 2b' + 1
+        *reinterpret_cast<uint2 *>(dst) = make_uint2(h0[0], h0[1]);
+        *reinterpret_cast<uint2 *>(dst + 4 * J * W) = make_uint2(l0[0], l0[1]);
       }
     }
   }
 }
 
-// Lanes (r = lane & 15, half = lane >> 4) decode one half of the scale groups of row r into the
-// warp's area; the corrections of the NB batch rows are combined across the halves by shuffles.
+// The J fragments (sets of four batch rows) of one lane and group, 8 bytes each.
+template <int J>
+__device__ __forceinline__ void load_sets(const uint8_t *p, uint2 (&bv)[J]) {
+  if constexpr (J == 2) {
+    const uint4 v = *reinterpret_cast<const uint4 *>(p);
+    bv[0] = make_uint2(v.x, v.y);
+    bv[1] = make_uint2(v.z, v.w);
+  } else {
+    bv[0] = *reinterpret_cast<const uint2 *>(p);
+  }
+}
+
+// Q8_0, IQ4_NL: lanes (r = lane & 15, half = lane >> 4) put the fp16 scales of one half of row r's
+// blocks into the warp's area.
 template <int TYPE, int NB>
-__device__ __forceinline__ void decode_dense(const uint8_t *blk_row, int lane, int kblk,
-                                             const float *XX, float *area) {
+__device__ __forceinline__ void decode_dense(const uint8_t *blk_row, int lane, float *area) {
   using C = Cfg<TYPE>;
-  constexpr int NH = C::NG / 2, ROW = dense_area_row(C::NG, NB);
+  constexpr int NH = C::NG / 2, ROW = dense_area_row(C::NG);
   const int r = lane & 15, half = lane >> 4;
   float dsc[NH], kk[NH];
   half_scales<TYPE>(blk_row, half, dsc, kk);
-  float *row = area + r * ROW;
-#pragma unroll
-  for (int i = 0; i < NH; i += 4)
-    *reinterpret_cast<float4 *>(row + NH * half + i) = make_float4(dsc[i], dsc[i + 1], dsc[i + 2], dsc[i + 3]);
-  if constexpr (C::HAS_MIN || TYPE == kQ6_K) {
-    float corr[NB];
-#pragma unroll
-    for (int b = 0; b < NB; b++) corr[b] = 0.f;
-    const float4 *xx = reinterpret_cast<const float4 *>(XX + (size_t)(kblk * C::NG + NH * half) * NB);
-#pragma unroll
-    for (int i = 0; i < NH; i++)
-#pragma unroll
-      for (int b4 = 0; b4 < NB / 4; b4++) {
-        const float4 c = xx[i * (NB / 4) + b4];
-        corr[4 * b4] = fmaf(kk[i], c.x, corr[4 * b4]);
-        corr[4 * b4 + 1] = fmaf(kk[i], c.y, corr[4 * b4 + 1]);
-        corr[4 * b4 + 2] = fmaf(kk[i], c.z, corr[4 * b4 + 2]);
-        corr[4 * b4 + 3] = fmaf(kk[i], c.w, corr[4 * b4 + 3]);
-      }
-#pragma unroll
-    for (int b = 0; b < NB; b++) {
-      corr[b] += __shfl_xor_sync(0xffffffffu, corr[b], 16);
-      if (TYPE == kQ6_K) corr[b] *= -32.f;
-    }
-    // the halves store alternate fours of the batch rows
-#pragma unroll
-    for (int b4 = 0; b4 < NB / 4; b4++)
-      if (half == (b4 & 1))
-        *reinterpret_cast<float4 *>(row + C::NG + 4 * b4) =
-            make_float4(corr[4 * b4], corr[4 * b4 + 1], corr[4 * b4 + 2], corr[4 * b4 + 3]);
-  } else {
-#pragma unroll
-    for (int b4 = 0; b4 < NB / 4; b4++)
-      if (half == (b4 & 1))
-        *reinterpret_cast<float4 *>(row + C::NG + 4 * b4) = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
+  *reinterpret_cast<float4 *>(area + r * ROW + NH * half) = make_float4(dsc[0], dsc[1], dsc[2], dsc[3]);
 }
 
-// MMAs of one superblock for all NB batch rows.  xg: this lane's B fragment of the superblock's
-// first (group, set); sxg: SX of the superblock's first group at batch row t.
+// MMAs of one superblock for all NB batch rows.  xg: this lane's B fragments of the superblock's
+// first group; sxg: SX of the superblock's first group at batch row t.
 template <int TYPE, int NB>
-__device__ __forceinline__ void mma_dense(const uint8_t *blk, int pad_a, int pad_b,
-                                          const uint8_t *xg, const float *area, const float *sxg,
-                                          int g, int t, float (&acc0)[NB / 4], float (&acc1)[NB / 4]) {
+__device__ __forceinline__ void mma_dense(const uint8_t *blk, const uint8_t *xg, const float *area,
+                                          const float *sxg, int g, int t, float (&acc0)[NB / 4],
+                                          float (&acc1)[NB / 4]) {
   using C = Cfg<TYPE>;
-  constexpr int J = NB / 4, GB = Dense<TYPE>::GB, ROW = dense_area_row(C::NG, NB);
-  constexpr uint32_t M4 = 0x0f0f0f0fu;
+  constexpr int J = NB / 4, GB = Dense<TYPE, NB>::GB, ROW = dense_area_row(C::NG);
   const float *rowa = area + g * ROW, *rowb = area + (g + 8) * ROW;
 #pragma unroll
-  for (int j = 0; j < J; j++) {
-    acc0[j] = rowa[C::NG + 4 * j + t];
-    acc1[j] = rowb[C::NG + 4 * j + t];
-  }
+  for (int j = 0; j < J; j++) acc0[j] = acc1[j] = 0.f;
   // scale group gi with A fragments (a0, a1, a2, a3): rows g / g+8, first / second eight elements
   auto group32 = [&](int gi, float fa, float fb, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
+    uint2 bv[J];
+    load_sets<J>(xg + gi * GB, bv);
 #pragma unroll
     for (int j = 0; j < J; j++) {
-      const uint2 bv = *reinterpret_cast<const uint2 *>(xg + (gi * J + j) * GB);
       int cc[4];
-      if constexpr (TYPE == kQ8_0 || TYPE == kIQ4_NL) imma_s8_zero(cc, a0, a1, a2, a3, bv.x, bv.y);
-      else imma_zero(cc, a0, a1, a2, a3, bv.x, bv.y);
+      imma_s8_zero(cc, a0, a1, a2, a3, bv[j].x, bv[j].y);
       const float sx = sxg[gi * NB + 4 * j];
       acc0[j] = fmaf(fa * sx, (float)(cc[0] * 128 + cc[1]), acc0[j]);
       acc1[j] = fmaf(fb * sx, (float)(cc[2] * 128 + cc[3]), acc1[j]);
@@ -940,7 +976,7 @@ __device__ __forceinline__ void mma_dense(const uint8_t *blk, int pad_a, int pad
       group32(2 * g4, sa.x, sb.x, lut4(wa0), lut4(wb0), lut4(wa0 >> 16), lut4(wb0 >> 16));
       group32(2 * g4 + 1, sa.y, sb.y, lut4(wa1), lut4(wb1), lut4(wa1 >> 16), lut4(wb1 >> 16));
     }
-  } else if constexpr (TYPE == kQ8_0) {
+  } else {
     const uint8_t *ra = blk + g * C::RS + 8 * t, *rb = blk + (g + 8) * C::RS + 8 * t;
     auto even_block = [](const uint8_t *p, uint32_t &w0, uint32_t &w1) {  // p: the block's d
       const uint32_t *q = reinterpret_cast<const uint32_t *>(p);
@@ -961,83 +997,6 @@ __device__ __forceinline__ void mma_dense(const uint8_t *blk, int pad_a, int pad
       group32(2 * g4, sa.x, sb.x, la0, lb0, la1, lb1);
       group32(2 * g4 + 1, sa.y, sb.y, ha[0], hb[0], ha[1], hb[1]);
     }
-  } else if constexpr (C::HAS_MIN) {
-    constexpr bool Q5 = TYPE == kQ5_K;
-    constexpr int QOFF = Q5 ? 48 : 16;
-    constexpr uint32_t M1 = 0x10101010u, MH = 0xf0f0f0f0u;
-    const uint8_t *ra = blk + g * C::RS + pad_a + 8 * t, *rb = blk + (g + 8) * C::RS + pad_b + 8 * t;
-    uint2 qha = make_uint2(0, 0), qhb = make_uint2(0, 0);
-    if constexpr (Q5) {
-      qha = *reinterpret_cast<const uint2 *>(ra + 16);
-      qhb = *reinterpret_cast<const uint2 *>(rb + 16);
-    }
-#pragma unroll 1  // rolled: the unrolled body of eight groups x two sets overflowed the instruction cache
-    for (int g4 = 0; g4 < 4; g4++) {
-      const float2 sa = *reinterpret_cast<const float2 *>(rowa + 2 * g4);
-      const float2 sb = *reinterpret_cast<const float2 *>(rowb + 2 * g4);
-      const uint2 qa = *reinterpret_cast<const uint2 *>(ra + QOFF + 32 * g4);
-      const uint2 qb = *reinterpret_cast<const uint2 *>(rb + QOFF + 32 * g4);
-      uint32_t la0 = qa.x & M4, la1 = qa.y & M4, lb0 = qb.x & M4, lb1 = qb.y & M4;
-      uint32_t ha0, ha1, hb0, hb1;
-      if constexpr (!Q5) {  // high nibbles stay in place: 16 * q, the 1/16 is in the group's scale
-        ha0 = qa.x & MH; ha1 = qa.y & MH; hb0 = qb.x & MH; hb1 = qb.y & MH;
-      } else {
-        ha0 = (qa.x >> 4) & M4; ha1 = (qa.y >> 4) & M4; hb0 = (qb.x >> 4) & M4; hb1 = (qb.y >> 4) & M4;
-        // fifth bit: bit 2*g4 of qh for the low-nibble elements, bit 2*g4+1 for the high ones
-        auto bit = [&](uint32_t q, int b) { return b <= 4 ? ((q << (4 - b)) & M1) : ((q >> (b - 4)) & M1); };
-        la0 |= bit(qha.x, 2 * g4);     la1 |= bit(qha.y, 2 * g4);
-        lb0 |= bit(qhb.x, 2 * g4);     lb1 |= bit(qhb.y, 2 * g4);
-        ha0 |= bit(qha.x, 2 * g4 + 1); ha1 |= bit(qha.y, 2 * g4 + 1);
-        hb0 |= bit(qhb.x, 2 * g4 + 1); hb1 |= bit(qhb.y, 2 * g4 + 1);
-      }
-      group32(2 * g4, sa.x, sb.x, la0, lb0, la1, lb1);
-      group32(2 * g4 + 1, sa.y, sb.y, ha0, hb0, ha1, hb1);
-    }
-  } else {
-    constexpr uint32_t M2 = 0x30303030u;
-    const uintptr_t aa = reinterpret_cast<uintptr_t>(blk + g * C::RS + pad_a + 4 * t);
-    const uintptr_t ab8 = reinterpret_cast<uintptr_t>(blk + (g + 8) * C::RS + pad_b + 4 * t);
-    const uint8_t *base[2] = {reinterpret_cast<const uint8_t *>(aa & ~(uintptr_t)3),
-                              reinterpret_cast<const uint8_t *>(ab8 & ~(uintptr_t)3)};
-    const uint32_t sh[2] = {(uint32_t)(aa & 2) * 8, (uint32_t)(ab8 & 2) * 8};
-#pragma unroll
-    for (int n = 0; n < 2; n++) {
-      const float4 sa0 = *reinterpret_cast<const float4 *>(rowa + 8 * n), sa1 = *reinterpret_cast<const float4 *>(rowa + 8 * n + 4);
-      const float4 sb0 = *reinterpret_cast<const float4 *>(rowb + 8 * n), sb1 = *reinterpret_cast<const float4 *>(rowb + 8 * n + 4);
-      const float sa[8] = {sa0.x, sa0.y, sa0.z, sa0.w, sa1.x, sa1.y, sa1.z, sa1.w};
-      const float sb[8] = {sb0.x, sb0.y, sb0.z, sb0.w, sb1.x, sb1.y, sb1.z, sb1.w};
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        uint32_t q[2][4];
-#pragma unroll
-        for (int r = 0; r < 2; r++) {
-          auto ld = [&](int off) {  // rows may start 2 bytes off a word: two loads and a funnel shift
-            const uint32_t *w32 = reinterpret_cast<const uint32_t *>(base[r] + off);
-            return __funnelshift_r(w32[0], w32[1], sh[r]);
-          };
-          const uint32_t ql0 = ld(64 * n + 16 * h), ql1 = ld(64 * n + 32 + 16 * h);
-          const uint32_t qhw = ld(128 + 32 * n + 16 * h);
-          q[r][0] = (ql0 & M4) | ((qhw << 4) & M2);
-          q[r][1] = (ql1 & M4) | ((qhw << 2) & M2);
-          q[r][2] = ((ql0 >> 4) & M4) | (qhw & M2);
-          q[r][3] = ((ql1 >> 4) & M4) | ((qhw >> 2) & M2);
-        }
-#pragma unroll
-        for (int k = 0; k < 4; k++) {  // elements 128n + 32k + 16h + (0..15): scale group 8n + 2k + h
-          const int gi = 8 * n + 2 * k + h;
-          const float fa = sa[2 * k + h], fb = sb[2 * k + h];
-#pragma unroll
-          for (int j = 0; j < J; j++) {
-            const uint32_t bw = *reinterpret_cast<const uint32_t *>(xg + (gi * J + j) * GB);
-            int cc[4];
-            imma16_zero(cc, q[0][k], q[1][k], bw);
-            const float sx = sxg[gi * NB + 4 * j];
-            acc0[j] = fmaf(fa * sx, (float)(cc[0] * 128 + cc[1]), acc0[j]);
-            acc1[j] = fmaf(fb * sx, (float)(cc[2] * 128 + cc[3]), acc1[j]);
-          }
-        }
-      }
-    }
   }
 }
 
@@ -1053,89 +1012,53 @@ __device__ __forceinline__ void mma_dense(const uint8_t *blk, int pad_a, int pad
 // offsets (-dmin * m, -32) are integer sums of (min or scale) x (group sum of n), below 5.4e8.
 template <int TYPE> constexpr bool kDenseInt = TYPE == kQ4_K || TYPE == kQ5_K || TYPE == kQ6_K;
 
-// Lanes (r = lane & 15, half = lane >> 4) write the integer scales of one half of row r's groups
-// into the warp's area; the offsets of the NB batch rows follow at index NG + b as floats.
-template <int TYPE, int NB>
-__device__ __forceinline__ void decode_dense_int(const uint8_t *blk_row, int lane, int kblk,
-                                                 const float *SX, const int *XN, float *area) {
-  using C = Cfg<TYPE>;
-  constexpr int NH = C::NG / 2, ROW = dense_area_row(C::NG, NB);
-  const int r = lane & 15, half = lane >> 4;
-  int sc[NH], mn[NH];
-  float dneg;  // the factor of the offset sum: -dmin, or -32 d
-  if constexpr (C::HAS_MIN) {
-    const uint4 h = *reinterpret_cast<const uint4 *>(blk_row);
-    dneg = -__high2float(*reinterpret_cast<const __half2 *>(&h.x));
-    const uint32_t u0 = h.y, u1 = h.z, u2 = h.w;
-    // four 6-bit scales / mins of this half as bytes (dequant.cr:240-249, four at a time)
-    const uint32_t scw = half ? ((u2 & 0x0f0f0f0fu) | ((u0 >> 2) & 0x30303030u)) : (u0 & 0x3f3f3f3fu);
-    const uint32_t mnw = half ? (((u2 >> 4) & 0x0f0f0f0fu) | ((u1 >> 2) & 0x30303030u)) : (u1 & 0x3f3f3f3fu);
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      sc[i] = (int)((scw >> (8 * i)) & 0xffu);
-      // Q4_K: the odd groups' sums arrive times 16 (nibbles in place), so the even ones' scales do
-      if (TYPE == kQ4_K && !(i & 1)) sc[i] <<= 4;
-      mn[i] = (int)((mnw >> (8 * i)) & 0xffu);
-    }
-  } else {
-    dneg = -32.f * load_half_as_float(blk_row + 208);
-    const int8_t *s8 = reinterpret_cast<const int8_t *>(blk_row + 192 + 8 * half);
-#pragma unroll
-    for (int i = 0; i < 8; i++) sc[i] = mn[i] = (int)s8[i];
-  }
-  int *row = reinterpret_cast<int *>(area + r * ROW);
-#pragma unroll
-  for (int i = 0; i < NH; i += 4)
-    *reinterpret_cast<int4 *>(row + NH * half + i) = make_int4(sc[i], sc[i + 1], sc[i + 2], sc[i + 3]);
-  int cs[NB];
-#pragma unroll
-  for (int b = 0; b < NB; b++) cs[b] = 0;
-  const int4 *xn = reinterpret_cast<const int4 *>(XN + (size_t)(kblk * C::NG + NH * half) * NB);
-#pragma unroll
-  for (int i = 0; i < NH; i++)
-#pragma unroll
-    for (int b4 = 0; b4 < NB / 4; b4++) {
-      const int4 c = xn[i * (NB / 4) + b4];
-      cs[4 * b4] += mn[i] * c.x;
-      cs[4 * b4 + 1] += mn[i] * c.y;
-      cs[4 * b4 + 2] += mn[i] * c.z;
-      cs[4 * b4 + 3] += mn[i] * c.w;
-    }
-#pragma unroll
-  for (int b = 0; b < NB; b++) cs[b] += __shfl_xor_sync(0xffffffffu, cs[b], 16);
-  // the halves store alternate fours of the batch rows
-#pragma unroll
-  for (int b4 = 0; b4 < NB / 4; b4++)
-    if (half == (b4 & 1)) {
-      const float4 sx = *reinterpret_cast<const float4 *>(SX + (size_t)kblk * NB + 4 * b4);
-      *reinterpret_cast<float4 *>(area + r * ROW + C::NG + 4 * b4) =
-          make_float4(dneg * sx.x * (float)cs[4 * b4], dneg * sx.y * (float)cs[4 * b4 + 1],
-                      dneg * sx.z * (float)cs[4 * b4 + 2], dneg * sx.w * (float)cs[4 * b4 + 3]);
-    }
-}
-
-// MMAs of one superblock for all NB batch rows.  xg: this lane's B fragment of the superblock's
-// first (group, set); sxb: the superblock's activation scales (one per batch row).
+// Every lane unpacks the scales of its own two rows from the header in registers (the four lanes of
+// a row do the same work, but an instruction of the warp costs the same for one lane as for all):
+// against scales decoded by two lanes per row into shared memory, with the offset sums as integer
+// multiply-adds, this takes a third of the instructions, no second pass over shared memory, and
+// leaves 25 KB more of it to the stages.  With the quantiser's wide stores, batch 8, us, before -> now:
+// Q4_K 12288 x 4096 16.3 -> 13.9, 34816 x 5120 57.3 -> 47.6; Q5_K 12288 x 4096 17.8 -> 15.2; Q6_K 12288 x
+// 4096 23.8 -> 19.5, 4096 x 4096 12.9 -> 10.1, 151936 x 4096 182 -> 152 (3.4 TB/s), and the 151936 x
+// 5120 head with its top-1 316 -> 181 (three stages fit now, two before).  Bound by the consumer warps:
+// 16 MMAs, 64 integer multiply-adds and 48 unpacking instructions a superblock are its core.
+//
+// MMAs of one superblock for all NB batch rows.  xg: this lane's B fragments of the superblock's
+// first group; xn: the superblock's group sums; sxb: its activation scales (one per batch row).
 template <int TYPE, int NB>
 __device__ __forceinline__ void mma_dense_int(const uint8_t *blk, int pad_a, int pad_b,
-                                              const uint8_t *xg, const float *area, const float *sxb,
+                                              const uint8_t *xg, const uint32_t *xn, const float *sxb,
                                               int g, int t, float (&acc0)[NB / 4], float (&acc1)[NB / 4]) {
   using C = Cfg<TYPE>;
-  constexpr int J = NB / 4, GB = Dense<TYPE>::GB, ROW = dense_area_row(C::NG, NB);
+  constexpr int J = NB / 4, GB = Dense<TYPE, NB>::GB, L = GroupSums<TYPE>::LANES;
   constexpr uint32_t M4 = 0x0f0f0f0fu;
-  const int *rowa = reinterpret_cast<const int *>(area + g * ROW);
-  const int *rowb = reinterpret_cast<const int *>(area + (g + 8) * ROW);
   int h0[J], l0[J], h1[J], l1[J];  // rows g / g+8, planes hi / lo, batch row 4j + t
 #pragma unroll
   for (int j = 0; j < J; j++) h0[j] = l0[j] = h1[j] = l1[j] = 0;
-  float da, db;
+  float da, db, na, nb;  // rows g / g+8: the factors of the sums and of the offset sums
+  uint32_t ca, cb;       // rows g / g+8: their A fragments (mins or scales) of the offset sums
   if constexpr (C::HAS_MIN) {
     constexpr bool Q5 = TYPE == kQ5_K;
     constexpr int QOFF = Q5 ? 48 : 16;
     constexpr uint32_t M1 = 0x10101010u, MH = 0xf0f0f0f0u;
     const uint8_t *ra = blk + g * C::RS + pad_a, *rb = blk + (g + 8) * C::RS + pad_b;
-    da = load_half_as_float(ra) * (Q5 ? 1.f : 0.0625f);
-    db = load_half_as_float(rb) * (Q5 ? 1.f : 0.0625f);
+    // the 6-bit scales of a row, 16 bits each: even / odd groups of the low / high four.  Q4_K: the
+    // odd groups' sums arrive times 16 (nibbles in place), so the even ones' scales do too.
+    uint32_t ev[2][2], od[2][2];
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      const uint4 h = *reinterpret_cast<const uint4 *>(r ? rb : ra);
+      const __half2 dd = *reinterpret_cast<const __half2 *>(&h.x);
+      (r ? db : da) = __low2float(dd) * (Q5 ? 1.f : 0.0625f);
+      (r ? nb : na) = -__high2float(dd);
+      // eight 6-bit scales / mins as bytes (dequant.cr:240-249, four at a time)
+      const uint32_t s0 = h.y & 0x3f3f3f3fu, s1 = (h.w & 0x0f0f0f0fu) | ((h.y >> 2) & 0x30303030u);
+      ev[r][0] = (s0 & 0x00ff00ffu) << (Q5 ? 0 : 4);
+      ev[r][1] = (s1 & 0x00ff00ffu) << (Q5 ? 0 : 4);
+      od[r][0] = (s0 >> 8) & 0x00ff00ffu;
+      od[r][1] = (s1 >> 8) & 0x00ff00ffu;
+      const uint32_t m0 = h.z & 0x3f3f3f3fu, m1 = ((h.w >> 4) & 0x0f0f0f0fu) | ((h.z >> 2) & 0x30303030u);
+      (r ? cb : ca) = t == 0 ? m0 : t == 1 ? m1 : 0u;  // k = 4t .. 4t+3, eight groups
+    }
     ra += 8 * t;
     rb += 8 * t;
     uint2 qha = make_uint2(0, 0), qhb = make_uint2(0, 0);
@@ -1144,21 +1067,21 @@ __device__ __forceinline__ void mma_dense_int(const uint8_t *blk, int pad_a, int
       qhb = *reinterpret_cast<const uint2 *>(rb + 16);
     }
     auto group32 = [&](int gi, int sa, int sb, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3) {
+      uint2 bv[J];
+      load_sets<J>(xg + gi * GB, bv);
 #pragma unroll
       for (int j = 0; j < J; j++) {
-        const uint2 bv = *reinterpret_cast<const uint2 *>(xg + (gi * J + j) * GB);
         int cc[4];
-        imma_zero(cc, a0, a1, a2, a3, bv.x, bv.y);
+        imma_zero(cc, a0, a1, a2, a3, bv[j].x, bv[j].y);
         h0[j] += sa * cc[0];
         l0[j] += sa * cc[1];
         h1[j] += sb * cc[2];
         l1[j] += sb * cc[3];
       }
     };
-#pragma unroll 1  // unrolling by 2 or 4 measured the same
+#pragma unroll
     for (int g4 = 0; g4 < 4; g4++) {
-      const int2 sa = *reinterpret_cast<const int2 *>(rowa + 2 * g4);
-      const int2 sb = *reinterpret_cast<const int2 *>(rowb + 2 * g4);
+      const int w = g4 >> 1, sh = 16 * (g4 & 1);  // groups 2 g4, 2 g4 + 1: halfword g4 & 1 of word w
       const uint2 qa = *reinterpret_cast<const uint2 *>(ra + QOFF + 32 * g4);
       const uint2 qb = *reinterpret_cast<const uint2 *>(rb + QOFF + 32 * g4);
       uint32_t la0 = qa.x & M4, la1 = qa.y & M4, lb0 = qb.x & M4, lb1 = qb.y & M4;
@@ -1174,63 +1097,99 @@ __device__ __forceinline__ void mma_dense_int(const uint8_t *blk, int pad_a, int
         ha0 |= bit(qha.x, 2 * g4 + 1); ha1 |= bit(qha.y, 2 * g4 + 1);
         hb0 |= bit(qhb.x, 2 * g4 + 1); hb1 |= bit(qhb.y, 2 * g4 + 1);
       }
-      group32(2 * g4, sa.x, sb.x, la0, lb0, la1, lb1);
-      group32(2 * g4 + 1, sa.y, sb.y, ha0, hb0, ha1, hb1);
+      group32(2 * g4, (int)((ev[0][w] >> sh) & 0xffffu), (int)((ev[1][w] >> sh) & 0xffffu), la0, lb0, la1, lb1);
+      group32(2 * g4 + 1, (int)((od[0][w] >> sh) & 0xffffu), (int)((od[1][w] >> sh) & 0xffffu), ha0, hb0, ha1, hb1);
     }
   } else {
     constexpr uint32_t M2 = 0x30303030u;
-    da = load_half_as_float(blk + g * C::RS + pad_a + 208);
-    db = load_half_as_float(blk + (g + 8) * C::RS + pad_b + 208);
-    const uintptr_t aa = reinterpret_cast<uintptr_t>(blk + g * C::RS + pad_a + 4 * t);
-    const uintptr_t ab8 = reinterpret_cast<uintptr_t>(blk + (g + 8) * C::RS + pad_b + 4 * t);
-    const uint8_t *base[2] = {reinterpret_cast<const uint8_t *>(aa & ~(uintptr_t)3),
-                              reinterpret_cast<const uint8_t *>(ab8 & ~(uintptr_t)3)};
-    const uint32_t sh[2] = {(uint32_t)(aa & 2) * 8, (uint32_t)(ab8 & 2) * 8};
+    const uint8_t *ra = blk + g * C::RS + pad_a, *rb = blk + (g + 8) * C::RS + pad_b;
+    da = load_half_as_float(ra + 208);
+    db = load_half_as_float(rb + 208);
+    na = -32.f * da;
+    nb = -32.f * db;
+    // rows may start 2 bytes off a word: two loads and a funnel shift
+    const uint8_t *base[2] = {reinterpret_cast<const uint8_t *>(reinterpret_cast<uintptr_t>(ra) & ~(uintptr_t)3),
+                              reinterpret_cast<const uint8_t *>(reinterpret_cast<uintptr_t>(rb) & ~(uintptr_t)3)};
+    const uint32_t sh[2] = {(uint32_t)(reinterpret_cast<uintptr_t>(ra) & 2) * 8, (uint32_t)(reinterpret_cast<uintptr_t>(rb) & 2) * 8};
+    auto body = [&](auto aligned) {  // aligned: no row of the warp is 2 bytes off
+      auto ld = [&](int r, int off) {
+        const uint32_t *w32 = reinterpret_cast<const uint32_t *>(base[r] + off);
+        if constexpr (decltype(aligned)::value) return w32[0];
+        else return __funnelshift_r(w32[0], w32[1], sh[r]);
+      };
 #pragma unroll
-    for (int n = 0; n < 2; n++) {
-      const int4 sa0 = *reinterpret_cast<const int4 *>(rowa + 8 * n), sa1 = *reinterpret_cast<const int4 *>(rowa + 8 * n + 4);
-      const int4 sb0 = *reinterpret_cast<const int4 *>(rowb + 8 * n), sb1 = *reinterpret_cast<const int4 *>(rowb + 8 * n + 4);
-      const int sa[8] = {sa0.x, sa0.y, sa0.z, sa0.w, sa1.x, sa1.y, sa1.z, sa1.w};
-      const int sb[8] = {sb0.x, sb0.y, sb0.z, sb0.w, sb1.x, sb1.y, sb1.z, sb1.w};
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        uint32_t q[2][4];
+      for (int n = 0; n < 2; n++) {
+        uint32_t sw[2][2];  // scales of groups 8n .. 8n+3, 8n+4 .. 8n+7
 #pragma unroll
         for (int r = 0; r < 2; r++) {
-          auto ld = [&](int off) {  // rows may start 2 bytes off a word: two loads and a funnel shift
-            const uint32_t *w32 = reinterpret_cast<const uint32_t *>(base[r] + off);
-            return __funnelshift_r(w32[0], w32[1], sh[r]);
-          };
-          const uint32_t ql0 = ld(64 * n + 16 * h), ql1 = ld(64 * n + 32 + 16 * h);
-          const uint32_t qhw = ld(128 + 32 * n + 16 * h);
-          q[r][0] = (ql0 & M4) | ((qhw << 4) & M2);
-          q[r][1] = (ql1 & M4) | ((qhw << 2) & M2);
-          q[r][2] = ((ql0 >> 4) & M4) | (qhw & M2);
-          q[r][3] = ((ql1 >> 4) & M4) | ((qhw >> 2) & M2);
+          sw[r][0] = ld(r, 192 + 8 * n);
+          sw[r][1] = ld(r, 196 + 8 * n);
         }
+        const int o = 64 * n + 4 * t, oh = 128 + 32 * n + 4 * t;
+        auto half = [&](auto hc) {
+          constexpr int h = decltype(hc)::value;
+          uint32_t q[2][4];
 #pragma unroll
-        for (int k = 0; k < 4; k++) {  // elements 128n + 32k + 16h + (0..15): scale group 8n + 2k + h
-          const int gi = 8 * n + 2 * k + h;
-#pragma unroll
-          for (int j = 0; j < J; j++) {
-            const uint32_t bw = *reinterpret_cast<const uint32_t *>(xg + (gi * J + j) * GB);
-            int cc[4];
-            imma16_zero(cc, q[0][k], q[1][k], bw);
-            h0[j] += sa[2 * k + h] * cc[0];
-            l0[j] += sa[2 * k + h] * cc[1];
-            h1[j] += sb[2 * k + h] * cc[2];
-            l1[j] += sb[2 * k + h] * cc[3];
+          for (int r = 0; r < 2; r++) {
+            const uint32_t ql0 = ld(r, o + 16 * h), ql1 = ld(r, o + 32 + 16 * h), qhw = ld(r, oh + 16 * h);
+            q[r][0] = (ql0 & M4) | ((qhw << 4) & M2);
+            q[r][1] = (ql1 & M4) | ((qhw << 2) & M2);
+            q[r][2] = ((ql0 >> 4) & M4) | (qhw & M2);
+            q[r][3] = ((ql1 >> 4) & M4) | ((qhw >> 2) & M2);
           }
-        }
+          auto group16 = [&](auto kc) {  // elements 128n + 32k + 16h + (0..15): scale group 8n + 2k + h
+            constexpr int k = decltype(kc)::value, i = 2 * k + h;
+            const int sa = sbyte<(i & 3)>(sw[0][i >> 2]), sb = sbyte<(i & 3)>(sw[1][i >> 2]);
+            const uint8_t *p = xg + (8 * n + i) * GB;
+            uint32_t bw[J];
+            if constexpr (J == 2) {
+              const uint2 v = *reinterpret_cast<const uint2 *>(p);
+              bw[0] = v.x;
+              bw[1] = v.y;
+            } else {
+              bw[0] = *reinterpret_cast<const uint32_t *>(p);
+            }
+#pragma unroll
+            for (int j = 0; j < J; j++) {
+              int cc[4];
+              imma16_zero(cc, q[0][k], q[1][k], bw[j]);
+              h0[j] += sa * cc[0];
+              l0[j] += sa * cc[1];
+              h1[j] += sb * cc[2];
+              l1[j] += sb * cc[3];
+            }
+          };
+          group16(std::integral_constant<int, 0>{});
+          group16(std::integral_constant<int, 1>{});
+          group16(std::integral_constant<int, 2>{});
+          group16(std::integral_constant<int, 3>{});
+        };
+        half(std::integral_constant<int, 0>{});
+        half(std::integral_constant<int, 1>{});
       }
-    }
+      ca = ld(0, 192 + 4 * t);  // groups 4t .. 4t+3
+      cb = ld(1, 192 + 4 * t);
+    };
+    if (__all_sync(0xffffffffu, (sh[0] | sh[1]) == 0)) body(std::true_type{});
+    else body(std::false_type{});
   }
-  const float *rowfa = area + g * ROW + C::NG, *rowfb = area + (g + 8) * ROW + C::NG;
+  int c0[4], c1[4], c2[4];  // offset sums, per plane of the group sums
+  const uint32_t *xw = C::HAS_MIN ? xn + 2 * g + (t & 1) : xn + 4 * g + t;  // (lanes t > 1 meet zeros in A)
+  if constexpr (C::HAS_MIN) {
+    imma16_zero(c0, ca, cb, xw[0]);
+    imma16_zero(c1, ca, cb, xw[L]);
+    imma16_zero(c2, ca, cb, xw[2 * L]);
+  } else {
+    imma16_s8_zero(c0, ca, cb, xw[0]);
+    imma16_s8_zero(c1, ca, cb, xw[L]);
+    imma16_s8_zero(c2, ca, cb, xw[2 * L]);
+  }
 #pragma unroll
   for (int j = 0; j < J; j++) {
     const float sx = sxb[4 * j + t];
-    acc0[j] = fmaf(da * sx, fmaf((float)h0[j], 128.f, (float)l0[j]), rowfa[4 * j + t]);
-    acc1[j] = fmaf(db * sx, fmaf((float)h1[j], 128.f, (float)l1[j]), rowfb[4 * j + t]);
+    const int oa = c0[j] + 128 * c1[j] + 16384 * c2[j], ob = c0[2 + j] + 128 * c1[2 + j] + 16384 * c2[2 + j];
+    acc0[j] = fmaf(da * sx, fmaf((float)h0[j], 128.f, (float)l0[j]), na * sx * (float)oa);
+    acc1[j] = fmaf(db * sx, fmaf((float)h1[j], 128.f, (float)l1[j]), nb * sx * (float)ob);
   }
 }
 
@@ -1297,8 +1256,7 @@ __device__ __forceinline__ void quantise_q6v2(const float *x, const float *x_up,
       float mx = 0.f;
 #pragma unroll
       for (int e = 0; e < 8; e++) mx = fmaxf(mx, fabsf(v[e]));
-#pragma unroll
-      for (int off = 1; off < 32; off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+      mx = warp_max_nonneg(mx);
       const bool live = mx > 1e-30f;  // a superblock below that contributes nothing
       const float sxb = live ? mx * (1.f / kNMax) : 1.f;
       const float inv = live ? (float)kNMax / mx : 0.f;
@@ -1433,7 +1391,7 @@ __global__ void __launch_bounds__((consumer_warps(TYPE, PAIR, NB) + kPW) * 32, 1
   constexpr int kFoldBufs = fold_bufs(NB);
   constexpr int NCX = 4 * NB;                    // columns of the quantised-x layout
   constexpr int UNIT_BYTES = NCX * 64;
-  constexpr int AREA_FLOATS = V2 ? 0 : DENSE ? 16 * dense_area_row(C::NG, NB) : PAIR * NB * A::BATCH;  // PAIR superblocks per item
+  constexpr int AREA_FLOATS = V2 || (DENSE && kDenseInt<TYPE>) ? 0 : DENSE ? 16 * dense_area_row(C::NG) : PAIR * NB * A::BATCH;  // PAIR superblocks per item
   extern __shared__ __align__(128) uint8_t smem[];
   // mbarriers full[S] | empty[S] in the first 128 bytes; monotone counters from byte 192:
   // chunks armed by the producer | partial sums stored per tile buffer | folds done per tile buffer
@@ -1588,7 +1546,7 @@ __global__ void __launch_bounds__((consumer_warps(TYPE, PAIR, NB) + kPW) * 32, 1
   const int npairs = (p.nblk + PAIR - 1) / PAIR;  // items per tile
   const int red_tile = npairs * 8 * NB;
   // this lane's 16 bytes of a unit's B fragments
-  const uint8_t *xlane = DENSE ? xq + lane * Dense<TYPE>::W : xq + ((g & (NCX - 1)) * 4 + t) * 16;
+  const uint8_t *xlane = DENSE ? xq + lane * (TYPE == kQ6_K ? 4 : 8) * (NB / 4) : xq + ((g & (NCX - 1)) * 4 + t) * 16;
   const uint32_t bar0 = smem_u32(bars);
 
   long long best = LLONG_MIN, best_b1 = LLONG_MIN;  // fused top-1: running maxima (batch row 0 / 1)
@@ -1661,15 +1619,13 @@ __global__ void __launch_bounds__((consumer_warps(TYPE, PAIR, NB) + kPW) * 32, 1
         constexpr int J = NB / 4;
         float acc0[J], acc1[J];  // rows g and g+8 of batch rows 4j + t
         if constexpr (kDenseInt<TYPE>) {
-          decode_dense_int<TYPE, NB>(blk + (lane & 15) * C::RS + pad_d, lane, e0, SX,
-                                     reinterpret_cast<const int *>(XX), area);
-          __syncwarp();
-          mma_dense_int<TYPE, NB>(blk, pad_a, pad_b, xlane + (size_t)e0 * C::NG * J * Dense<TYPE>::GB,
-                                  area, SX + (size_t)e0 * NB, g, t, acc0, acc1);
+          mma_dense_int<TYPE, NB>(blk, pad_a, pad_b, xlane + (size_t)e0 * C::NG * Dense<TYPE, NB>::GB,
+                                  reinterpret_cast<const uint32_t *>(XX) + (size_t)e0 * GroupSums<TYPE>::WORDS,
+                                  SX + (size_t)e0 * NB, g, t, acc0, acc1);
         } else {
-          decode_dense<TYPE, NB>(blk + (lane & 15) * C::RS + pad_d, lane, e0, XX, area);
+          decode_dense<TYPE, NB>(blk + (lane & 15) * C::RS, lane, area);
           __syncwarp();
-          mma_dense<TYPE, NB>(blk, pad_a, pad_b, xlane + (size_t)e0 * C::NG * J * Dense<TYPE>::GB, area,
+          mma_dense<TYPE, NB>(blk, xlane + (size_t)e0 * C::NG * Dense<TYPE, NB>::GB, area,
                               SX + (size_t)e0 * C::NG * NB + t, g, t, acc0, acc1);
         }
         __syncwarp();  // the area is rewritten by this warp's next decode
@@ -1942,12 +1898,17 @@ bool make_plan_pair(int in_dim, int nb, int pair, Params &p, size_t &smem, bool 
   const size_t off_flags = off;  off += (size_t)nflags * 4;
   const bool dense = nb > 2;  // nb = 4 or 8 then: single-superblock items, 2 bytes of x per element and batch row
   const bool v2 = TYPE == kQ6_K && !dense;  // Q6_K batch 1-2: no decode areas, 2 bytes of x per element and batch row
-  const size_t area_floats = v2 ? 0 : dense ? (size_t)16 * dense_area_row(C::NG, nb) : (size_t)pair * nb * Area<TYPE>::BATCH;
+  const bool dense_int = dense && kDenseInt<TYPE>;  // scales unpacked in registers
+  const size_t area_floats = v2 || dense_int ? 0 : dense ? (size_t)16 * dense_area_row(C::NG) : (size_t)pair * nb * Area<TYPE>::BATCH;
   const size_t off_red = off;    off = al(off + (size_t)fold_bufs(nb) * ((nblk + pair - 1) / pair) * 8 * nb * 8);  // [tile buffer][item][g][batch] float2
   const size_t off_area = off;   off = al(off + (size_t)consumer_warps(TYPE, pair, nb) * area_floats * 4);
-  const size_t off_sx = off;     off = al(off + (size_t)ngroups * nb * 4);
-  const size_t off_xx = off;     off = al(off + (size_t)ngroups * nb * 4);
-  const size_t off_xq = off;     off = al(off + (dense || v2 ? (size_t)in_dim * 2 * nb : (size_t)(in_dim / 64) * (4 * nb) * 64));
+  const size_t off_sx = off;     off = al(off + (size_t)(dense_int ? nblk : ngroups) * nb * 4);
+  const size_t off_xx = off;
+  off = al(off + (dense_int ? (size_t)nblk * GroupSums<TYPE>::WORDS * 4 : dense ? 0 : (size_t)ngroups * nb * 4));
+  const size_t off_xq = off;
+  off = al(off + (dense ? (size_t)ngroups * (nb == 4 ? Dense<TYPE, 4>::GB : Dense<TYPE, 8>::GB)
+                  : v2  ? (size_t)in_dim * 2 * nb
+                        : (size_t)(in_dim / 64) * (4 * nb) * 64));
   const size_t off_stage = off;
   const size_t stage_bytes = al((size_t)kR * C::RS);
   // Three stages, or for the 4- and 8-row instances two that still keep 64 KB in flight (Q5_K
@@ -2018,7 +1979,7 @@ int launch_instance(const Params &p, size_t smem, int grid, cudaStream_t s) {
 }
 
 // Batch rows of the kernel instance that takes `batch` (<= 8) rows: 1, 2, 4 or 8; IQ4_NL has only
-// the 4- and 8-row instances (unused rows repeat the last one).
+// the 4- and 8-row instances.
 template <int TYPE>
 int kernel_rows(int batch) {
   if (batch <= 2 && TYPE != kIQ4_NL) return batch;
