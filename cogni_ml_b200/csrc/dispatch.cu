@@ -2,6 +2,7 @@
 #include <climits>
 
 #include "qmm_common.cuh"
+#include "tma_pipe.cuh"
 
 namespace cogni {
 
@@ -103,6 +104,10 @@ __global__ void __launch_bounds__(kTop2Threads)
   const int b = blockIdx.y, part = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float *row = logits + (long long)b * out_dim;
   KeyPair p{LLONG_MIN, LLONG_MIN};
+  // launched while the GEMV that writes the logits still runs: its last CTA's end, not a launch, is
+  // what the first load waits for
+  pdl_wait_prior_grid();
+#pragma unroll 4
   for (int i = part * kTop2Threads + threadIdx.x; i < out_dim; i += nparts * kTop2Threads)
     pair_insert(p, top1_key(row[i], (uint32_t)(index_base + i)));
   auto block_merge = [&](KeyPair &q) {
@@ -174,9 +179,17 @@ int launch_gemv_top2(int type, const void *d_w, const float *d_x, int in_dim, in
                                logits + (long long)b0 * out_dim, in_dim, out_dim, nb, resident, s);
     if (st) return st;
   }
-  top2_scan_kernel<<<dim3(nparts, batch), kTop2Threads, 0, s>>>(logits, out_dim, index_base, ctr, parts,
-                                                               nparts, d_idx, d_val, d_key);
-  return (int)cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(nparts, batch);
+  cfg.blockDim = dim3(kTop2Threads);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, top2_scan_kernel, (const float *)logits, out_dim, index_base, ctr, parts,
+                                 nparts, d_idx, d_val, d_key);
 }
 
 int launch_rmsnorm(const float *d_x, const float *d_w, float eps, float *d_out, int rows, int dim,
