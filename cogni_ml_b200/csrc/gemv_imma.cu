@@ -1375,13 +1375,16 @@ __device__ __forceinline__ void mma_q6v2(const uint8_t *ra, const uint8_t *rb, c
 // VAR picks how much the instance carries: 0 the plain GEMV; 1 adds the fused prologues (RMSNorm,
 // SwiGLU) to the activation quantisers; 2 also splits row tiles over K slabs, exchanges its outputs
 // with the other GPUs and reads activations that come out of an exchange; 3 is the plain GEMV that
-// only sends its outputs (whole rows, plain activations).  The plain instance carries none of
+// only sends its outputs (whole rows, plain activations); 4 is 1 with K slabs and no exchange (batch
+// 8, us, on instance 2 / 4: Q6_K 4096 x 12288 29.1 / 25.0, 5120 x 17408 with SwiGLU 65.2 / 54.6, Q4_K
+// 4096 x 12288 25.3 / 23.1: a fifth of the spilled registers).  The plain instance carries none of
 // that code.
 template <int TYPE, int NB, int PAIR, int VAR>
 __global__ void __launch_bounds__((consumer_warps(TYPE, PAIR, NB) + kPW) * 32, 1)
     gemv_imma_kernel(const Params p) {
-  // XT: K slabs and exchanged activations; XO: outputs go to the other GPUs
-  constexpr bool XT = VAR == 2, XO = VAR >= 2, PRO = VAR == 1 || VAR == 2;
+  // XS: K slabs; XL: exchanged activations; XO: outputs go to the other GPUs
+  constexpr bool XS = VAR == 2 || VAR == 4, XL = VAR == 2, XO = VAR == 2 || VAR == 3;
+  constexpr bool PRO = VAR == 1 || VAR == 2 || VAR == 4;
   constexpr int kNW = consumer_warps(TYPE, PAIR, NB), kThreads = (kNW + kPW) * 32;
   using C = Cfg<TYPE>;
   using A = Area<TYPE>;
@@ -1406,7 +1409,7 @@ __global__ void __launch_bounds__((consumer_warps(TYPE, PAIR, NB) + kPW) * 32, 1
   uint8_t *stages = smem + p.off_stage;
   // The jobs' 16-row tiles form one global sequence (job-major).  The grid is G row groups x
   // nslabs K slabs: this CTA takes slab `slab` of the tiles rg + i * G, i < ntl.
-  const int nslabs = XT ? p.nslabs : 1;
+  const int nslabs = XS ? p.nslabs : 1;
   const int slab = nslabs > 1 ? (int)blockIdx.x % nslabs : 0;
   const int rg = nslabs > 1 ? (int)blockIdx.x / nslabs : (int)blockIdx.x;
   const int G = nslabs > 1 ? (int)gridDim.x / nslabs : (int)gridDim.x;
@@ -1504,7 +1507,7 @@ __global__ void __launch_bounds__((consumer_warps(TYPE, PAIR, NB) + kPW) * 32, 1
       }
     }
   }
-  const XSrc xsrc{XT ? p.ex_wait : 0, ex_epoch};
+  const XSrc xsrc{XL ? p.ex_wait : 0, ex_epoch};
 
   // RMSNorm prologue: 1 / sqrt(mean(x^2) + eps) per batch row, the sum of squares in f64 as the
   // reference has it (qwen35_cpu.cr:484-490); per-warp partial sums are added in warp order, so
@@ -1520,7 +1523,7 @@ __global__ void __launch_bounds__((consumer_warps(TYPE, PAIR, NB) + kPW) * 32, 1
       const int br = DENSE ? min(b, p.batch - 1) : b;
       double ss = 0.0;
       for (int k = ctid * 4; k < p.norm_dim; k += kNW * 32 * 4) {
-        const float4 v = XT && xsrc.ll ? ld4x<true>(p.norm_x, (long long)br * K + k, xsrc)
+        const float4 v = XL && xsrc.ll ? ld4x<true>(p.norm_x, (long long)br * K + k, xsrc)
                                        : ld4x<false>(p.norm_x, (long long)br * K + k, xsrc);
         ss += (double)v.x * v.x + (double)v.y * v.y + (double)v.z * v.z + (double)v.w * v.w;
       }
@@ -1600,7 +1603,7 @@ __global__ void __launch_bounds__((consumer_warps(TYPE, PAIR, NB) + kPW) * 32, 1
             else quantise_superblocks<TYPE, NB, 1, LL>(xs, xs_up, norm_ws, s_inv_rms, K, e0, lane, xq, SX, XX, xsrc);
           }
         };
-        if constexpr (XT) {
+        if constexpr (XL) {
           if (xsrc.ll) quantise(std::true_type{});
           else quantise(std::false_type{});
         } else {
@@ -1735,7 +1738,7 @@ __global__ void __launch_bounds__((consumer_warps(TYPE, PAIR, NB) + kPW) * 32, 1
         }
         __syncwarp();
         if (lane == 0) st_release_shared(&folded[tb], fl / kFoldBufs + 1);
-        if (XT && nslabs > 1) {
+        if (XS && nslabs > 1) {
           float *part = p.ws + (((long long)gt * nslabs + slab) * NB + (lane >> 4)) * 16 + r16;
 #pragma unroll
           for (int i = 0; i < NB / 2; i++) part[2 * i * 16] = v[i];
@@ -1778,7 +1781,7 @@ __global__ void __launch_bounds__((consumer_warps(TYPE, PAIR, NB) + kPW) * 32, 1
       for (int k = 0; k < npairs; k++) v += src[k * 16 * NB];
       __syncwarp();
       if (lane == 0) st_release_shared(&folded[tb], fl / kFoldBufs + 1);
-      if (XT && nslabs > 1) {
+      if (XS && nslabs > 1) {
         if (b < NB) p.ws[(((long long)gt * nslabs + slab) * NB + b) * 16 + r16] = v;
         slab_ticket();
         if (last_slab) {
@@ -1971,6 +1974,8 @@ int launch_instance_x(const Params &p, size_t smem, int grid, cudaStream_t s) {
 }
 template <int TYPE, int NB, int PAIR>
 int launch_instance(const Params &p, size_t smem, int grid, cudaStream_t s) {
+  if (p.nslabs > 1 && !p.ex_wait && !p.ex.epoch && !p.y_pitch)
+    return launch_instance_x<TYPE, NB, PAIR, 4>(p, smem, grid, s);
   if (p.nslabs > 1 || p.ex_wait || (p.ex.world > 1 && (p.x_up || p.norm_w)))
     return launch_instance_x<TYPE, NB, PAIR, 2>(p, smem, grid, s);
   if (p.ex.world > 1) return launch_instance_x<TYPE, NB, PAIR, 3>(p, smem, grid, s);
