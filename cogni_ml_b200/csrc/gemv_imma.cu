@@ -59,11 +59,11 @@ namespace {
 // more warps leave fewer stages for the copies in flight; 16 (20 for single-superblock items of
 // the 210-byte Q6_K blocks) measured best for batches 1-2.  The 4- and 8-row instances are bound
 // by their consumer warps' latencies and take 20 (batch 8: Q4_K 65536 x 4096 55.4 -> 51.5 us,
-// 4096 x 16384 32.6 -> 27.2, Q5_K 65536 x 4096 69.6 -> 60.5; 24 warps: Q4_K 53.2), except Q6_K,
-// whose slab launches need the stages (4096 x 12288 with 20: 29.3 -> 31.4 us, the 151936 x 5120
-// head 262 -> 278).
+// 4096 x 16384 32.6 -> 27.2, Q5_K 65536 x 4096 69.6 -> 60.5; 24 warps: Q4_K 53.2).  Q6_K, with 16 / 20:
+// 5120 x 17408 with SwiGLU 54.6 / 41.6, 4096 x 8192 22.4 / 19.7, 151936 x 4096 151 / 140, 12288 x 4096
+// 19.5 / 19.1, but 4096 x 12288 25.0 / 26.2 and 4096 x 4096 10.0 / 10.4.
 __host__ __device__ constexpr int consumer_warps(int type, int pair, int nb = 1) {
-  if (nb > 2) return type == kQ6_K ? 16 : 20;
+  if (nb > 2) return 20;
   return type == kQ6_K && pair == 1 ? 20 : 16;
 }
 // tiles whose partial sums can be pending (power of 2)
