@@ -220,7 +220,8 @@ __global__ void __launch_bounds__(kBlockWarps * 32)
   const int nblk = in_dim >> 5;
   const int kw = warp & (wk - 1), grp = warp / wk;  // this warp's part of K, its row group of the CTA
   const int row0 = ((int)(blockIdx.x / bgroups) * (kBlockWarps / wk) + grp) * RPW;
-  const int b0 = min((int)(blockIdx.x % bgroups) * NB, batch - NB);  // the last group overlaps the one before
+  const int first = (int)(blockIdx.x % bgroups) * NB;  // the columns that this group stores start here
+  const int b0 = min(first, batch - NB);               // the last group computes some of the one before again
   const long long row_bytes = (long long)nblk * BB;
   const uint8_t *wr[RPW];
 #pragma unroll
@@ -281,7 +282,8 @@ __global__ void __launch_bounds__(kBlockWarps * 32)
     float sum = 0.f;
     for (int k = 0; k < wk; k++) sum += s_part[g * wk + k][i];
     const int b = b0 + c;
-    if (c < NB && row < out_dim) {
+    // One CTA per output: the addend may be y itself, and a second one would add onto the first's result.
+    if (c < NB && b >= first && row < out_dim) {
       const float a = addend ? addend[(int64_t)b * addend_stride + row] : 0.f;
       y[(int64_t)b * out_dim + row] = a + sum;
     }

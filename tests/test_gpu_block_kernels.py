@@ -44,6 +44,29 @@ def test_gemv_of_whole_blocks(cuda, oracle, qtype, batch, out_dim, in_dim):
     assert np.abs(dw.gemv(xo).cpu().numpy() - ref).max() <= 1e-5 * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("qtype,out_dim,in_dim,slabs", [
+    (Q8_0, 700, 2976, 0), (IQ4_NL, 700, 2976, 0), (Q8_0, 9001, 288, 0), (IQ4_NL, 9001, 288, 0),  # block kernel
+    (Q4_K, 700, 1024, 0), (IQ4_NL, 700, 1024, 0), (Q4_K, 597, 4096, 4), (Q6_K, 597, 12288, 3)])  # tiled, K slabs
+def test_residual_in_place(cuda, engine, qtype, out_dim, in_dim, slabs):
+    """The addend may be the output itself: the bits of a call with a separate residual, whatever the
+    batch (groups of columns that do not divide it) and however often.  No oracle: both calls add the
+    same sums."""
+    w = synth.make_weight(qtype, out_dim, in_dim, seed=47, tensor_id=qtype)
+    dw = DeviceQuantWeight.upload(QuantWeight(w, qtype, out_dim, in_dim), cuda)
+    engine.lib.cogni_qmm_set_kernel_choice(60 + slabs)
+    try:
+        for batch in [*range(3, 17), 21]:
+            x = torch.from_numpy(synth.make_activation(batch, in_dim, seed=47)).to(cuda)
+            res = torch.from_numpy(synth.make_activation(batch, out_dim, 47, 5)).to(cuda)
+            want = dw.gemv(x, residual=res)
+            for _ in range(10):
+                h = res.clone()
+                dw.gemv(x, out=h, residual=h)
+                assert torch.equal(h, want), f"batch {batch}: {int((h != want).sum())} values differ"
+    finally:
+        engine.lib.cogni_qmm_set_kernel_choice(60)
+
+
 @pytest.mark.parametrize("qtype", [Q8_0, Q4_K, Q5_K, Q6_K, IQ4_NL])
 @pytest.mark.parametrize("blocks", [1, 7, 33, 129])
 @pytest.mark.parametrize("w_at,y_at", [(0, 0), (2, 0), (0, 4)])
