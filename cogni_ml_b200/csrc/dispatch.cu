@@ -156,22 +156,24 @@ __global__ void __launch_bounds__(kTop2Threads)
 }
 }  // namespace
 
-// scratch: counters[batch] (8-byte aligned total) | part keys [batch][nparts][2] | logits [batch][out_dim]
+// scratch: kTop2Rows ticket counters | part keys [batch][nparts][2] | logits [batch][out_dim].  The counters
+// alone carry something (zero) from call to call, so their place depends on nothing: calls of any batch
+// and out_dim that a scratch buffer is large enough for may follow each other on it.  A launch of the scan
+// takes as many rows as there are counters.
+constexpr int kTop2Rows = 64;
 int top2_parts(int out_dim) {
   const int want = (out_dim + kTop2Threads * 8 - 1) / (kTop2Threads * 8);
   return want < 1 ? 1 : (want > 592 ? 592 : want);
 }
 size_t top2_scratch_bytes(int out_dim, int batch) {
-  const size_t counters = ((size_t)batch * 4 + 7) & ~(size_t)7;
-  return counters + (size_t)batch * top2_parts(out_dim) * 16 + (size_t)batch * out_dim * 4;
+  return kTop2Rows * sizeof(unsigned) + (size_t)batch * top2_parts(out_dim) * 16 + (size_t)batch * out_dim * 4;
 }
 int launch_gemv_top2(int type, const void *d_w, const float *d_x, int in_dim, int out_dim, int batch,
                      int32_t index_base, void *d_scratch, int32_t *d_idx, float *d_val,
                      long long *d_key, int resident, cudaStream_t s) {
   const int nparts = top2_parts(out_dim);
-  const size_t counters = ((size_t)batch * 4 + 7) & ~(size_t)7;
   unsigned *ctr = static_cast<unsigned *>(d_scratch);
-  long long *parts = reinterpret_cast<long long *>(static_cast<char *>(d_scratch) + counters);
+  long long *parts = reinterpret_cast<long long *>(ctr + kTop2Rows);
   float *logits = reinterpret_cast<float *>(parts + (size_t)batch * nparts * 2);
   for (int b0 = 0; b0 < batch; b0 += 16) {  // the GEMV kernels take up to 16 rows a call
     const int nb = batch - b0 < 16 ? batch - b0 : 16;
@@ -180,7 +182,6 @@ int launch_gemv_top2(int type, const void *d_w, const float *d_x, int in_dim, in
     if (st) return st;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(nparts, batch);
   cfg.blockDim = dim3(kTop2Threads);
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -188,8 +189,14 @@ int launch_gemv_top2(int type, const void *d_w, const float *d_x, int in_dim, in
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, top2_scan_kernel, (const float *)logits, out_dim, index_base, ctr, parts,
-                                 nparts, d_idx, d_val, d_key);
+  for (int b0 = 0; b0 < batch; b0 += kTop2Rows) {
+    cfg.gridDim = dim3(nparts, batch - b0 < kTop2Rows ? batch - b0 : kTop2Rows);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, top2_scan_kernel, (const float *)logits + (long long)b0 * out_dim, out_dim,
+                                             index_base, ctr, parts + (long long)b0 * nparts * 2, nparts, d_idx + 2 * b0,
+                                             d_val + 2 * b0, d_key ? d_key + 2 * b0 : nullptr);
+    if (e != cudaSuccess) return (int)e;
+  }
+  return COGNI_QMM_OK;
 }
 
 int launch_rmsnorm(const float *d_x, const float *d_w, float eps, float *d_out, int rows, int dim,

@@ -189,7 +189,8 @@ int cogni_qmm_gemv_top1_rmsnorm(int type, const void *d_w, const float *d_x,
  * output_top2_partial_scan_probe / output_top2_partial_reduce_probe
  * (src/ml/cuda/qwen_output_head_runner.cr:158-338, 864-904).  out_dim >= 2.  The scratch buffer
  * (cogni_qmm_gemv_top2_scratch_bytes, 8-byte aligned) must be zero-filled once before its first
- * use; the logits stay readable in it after the call, f32 [batch, out_dim] at its end.
+ * use; calls of any batch and out_dim that it is large enough for may then follow each other on it.
+ * The logits stay readable in it after the call, f32 [batch, out_dim] at the end of these bytes.
  */
 size_t cogni_qmm_gemv_top2_scratch_bytes(int out_dim, int batch);
 int cogni_qmm_gemv_top2(int type, const void *d_w, const float *d_x, int in_dim, int out_dim,

@@ -388,6 +388,31 @@ def test_lm_head_top2_and_margin(cuda, oracle, qtype, batch):
     assert torch.equal(i1, idx[:, 0].contiguous()) or batch > 2   # batch > 2 takes another GEMV kernel
 
 
+@pytest.mark.parametrize("qtype,out_dim,in_dim", [(Q6_K, 5003, 1024), (IQ4_NL, 2048, 288), (Q4_K, 301, 512)])
+def test_lm_head_top2_scratch_serves_every_batch(cuda, oracle, engine, qtype, out_dim, in_dim):
+    """One scratch buffer, zero-filled once, serves calls of changing batch (and fewer rows of the matrix):
+    a smaller batch must leave nothing that a larger one takes for its tickets.  70 rows are two scans."""
+    lib, largest = engine.lib, 70
+    w = synth.make_weight(qtype, out_dim, in_dim, seed=67, tensor_id=qtype)
+    x = synth.make_activation(largest, in_dim, seed=67)
+    dw = DeviceQuantWeight.upload(QuantWeight(w, qtype, out_dim, in_dim), cuda)
+    xd = torch.from_numpy(x).to(cuda)
+    logits = oracle.matmul_add(x, largest, in_dim, w, qtype, out_dim, np.zeros(out_dim, np.float32),
+                               threads=oracle.max_threads()).reshape(largest, out_dim)
+    size = lib.cogni_qmm_gemv_top2_scratch_bytes(out_dim, largest)
+    scratch = torch.zeros(size, dtype=torch.uint8, device=cuda)
+    for batch, n in [(5, out_dim), (1, out_dim), (5, out_dim), (16, out_dim), (2, out_dim - 3), (70, out_dim), (3, 300), (9, out_dim)]:
+        idx = torch.full((batch, 2), -1, dtype=torch.int32, device=cuda)
+        val = torch.full((batch, 2), float("nan"), device=cuda)
+        st = lib.cogni_qmm_gemv_top2(qtype, dw.raw.data_ptr(), xd.data_ptr(), in_dim, n, batch, 0, scratch.data_ptr(), size,
+                                     idx.data_ptr(), val.data_ptr(), None, 0, torch.cuda.current_stream().cuda_stream)
+        assert st == 0
+        best = -np.sort(-logits[:batch, :n], axis=1)[:, :2]
+        assert np.abs(val.cpu().numpy() - best).max() <= REL_TOL * np.abs(logits).max(), f"batch {batch}"
+        at = np.take_along_axis(logits[:batch, :n], idx.cpu().numpy().astype(np.int64), 1)
+        assert np.abs(at - best).max() <= 2 * REL_TOL * np.abs(logits).max(), f"batch {batch}"
+
+
 def test_lm_head_top2_tie_takes_the_two_lowest_indices(cuda):
     in_dim, out_dim = 256, 300
     row = synth.make_weight(Q6_K, 1, in_dim, seed=71)
