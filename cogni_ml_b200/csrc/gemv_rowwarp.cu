@@ -419,6 +419,10 @@ int run_top1(const void *d_w, const float *d_x, int in_dim, int out_dim, int bat
   unsigned *counters = static_cast<unsigned *>(d_scratch);
   long long *keys = reinterpret_cast<long long *>(static_cast<char *>(d_scratch) +
                                                   (((size_t)batch * 4 + 7) & ~(size_t)7));
+  // A call of a smaller batch, or of the tiled kernel (one counter), on the same scratch buffer has its
+  // part keys where this one's counters lie.
+  const cudaError_t e = cudaMemsetAsync(counters, 0, (size_t)batch * sizeof(unsigned), s);
+  if (e != cudaSuccess) return (int)e;
   dim3 grid(nparts, batch), block(kWarpsPerCta * 32);
   gemv_top1_rowwarp_kernel<TYPE><<<grid, block, 0, s>>>(static_cast<const uint8_t *>(d_w), d_x,
                                                          in_dim, out_dim, index_base, counters,

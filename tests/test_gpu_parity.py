@@ -423,6 +423,31 @@ def test_lm_head_top2_tie_takes_the_two_lowest_indices(cuda):
     assert idx[0].tolist() == [0, 1] and float(val[0, 0]) == float(val[0, 1])
 
 
+@pytest.mark.parametrize("qtype,out_dim,in_dim", [(Q8_0, 3001, 288), (Q6_K, 3001, 1024)])
+def test_lm_head_top1_scratch_serves_every_batch(cuda, oracle, engine, qtype, out_dim, in_dim):
+    """As for the top-2, and with the two kernels in turn (an unaligned x takes the row-per-warp one)."""
+    lib, largest = engine.lib, 16
+    w = synth.make_weight(qtype, out_dim, in_dim, seed=69, tensor_id=qtype)
+    x = synth.make_activation(largest, in_dim, seed=69)
+    dw = DeviceQuantWeight.upload(QuantWeight(w, qtype, out_dim, in_dim), cuda)
+    xd = torch.from_numpy(x).to(cuda)
+    off = torch.empty(x.size + 4, device=cuda)[1:x.size + 1].copy_(xd.view(-1))
+    logits = oracle.matmul_add(x, largest, in_dim, w, qtype, out_dim, np.zeros(out_dim, np.float32),
+                               threads=oracle.max_threads()).reshape(largest, out_dim)
+    size = lib.cogni_qmm_gemv_top1_scratch_bytes(out_dim, largest)
+    scratch = torch.zeros(size, dtype=torch.uint8, device=cuda)
+    for batch, rows in [(5, xd), (1, xd), (5, off), (2, off), (16, off), (5, xd), (4, off)]:
+        idx = torch.full((batch,), -1, dtype=torch.int32, device=cuda)
+        val = torch.full((batch,), float("nan"), device=cuda)
+        st = lib.cogni_qmm_gemv_top1(qtype, dw.raw.data_ptr(), rows.data_ptr(), in_dim, out_dim, batch, 0, scratch.data_ptr(),
+                                     size, idx.data_ptr(), val.data_ptr(), None, torch.cuda.current_stream().cuda_stream)
+        assert st == 0
+        best = logits[:batch].max(1)
+        assert np.abs(val.cpu().numpy() - best).max() <= REL_TOL * np.abs(logits).max(), f"batch {batch}"
+        at = np.take_along_axis(logits[:batch], idx.cpu().numpy().astype(np.int64)[:, None], 1)[:, 0]
+        assert np.abs(at - best).max() <= 2 * REL_TOL * np.abs(logits).max(), f"batch {batch}"
+
+
 @pytest.mark.parametrize("qtype,batch", [(Q6_K, 1), (Q4_K, 2), (Q8_0, 1), (Q6_K, 5), (Q4_K, 8),
                                          (Q5_K, 12), (Q8_0, 3)])
 def test_lm_head_top1_with_fused_output_norm(cuda, oracle, qtype, batch):
