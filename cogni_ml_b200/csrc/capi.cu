@@ -4,6 +4,7 @@
 #include <cstdio>
 #include <cstring>
 
+#include "host_workspace.cuh"
 #include "qmm_common.cuh"
 #include "../../include/cogni_qmm_diag.h"
 

@@ -5,11 +5,16 @@
 // against 0.55 ms for the copy of a 9.4 MB weight: blocks are therefore kept, up to kKeepBytes and
 // kSlots in all, and handed from call to call.  A block belongs to one call at a time (several
 // threads get several blocks) and to the CUDA context that it was allocated in; nothing of its content
-// is ever read by a later call.  cogni_qmm_release_host_workspaces gives the idle ones back.
+// is ever read by a later call.  cogni_qmm_release_host_workspaces gives the idle ones back, and so does
+// a call for which the device has no memory left.
+//
+// Host code only (no kernels, nothing but the runtime's C API): tests/cpp runs it on a CPU against a
+// device that is made up.
+#include "host_workspace.cuh"
+
 #include <cuda.h>
 #include <mutex>
 
-#include "qmm_common.cuh"
 
 namespace cogni {
 namespace {
@@ -47,6 +52,27 @@ unsigned long long context_id() {
   return id;
 }
 
+// Gives the idle blocks of context `ctx` (the current one) back; their number in *count.
+cudaError_t release_idle(unsigned long long ctx, int *count) {
+  void *idle[kSlots];
+  int n = 0;
+  {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    for (Slot &s : g_slots)
+      if (s.bytes && !s.lent && s.ctx == ctx) {
+        idle[n++] = s.p;
+        s = Slot{};
+      }
+  }
+  cudaError_t first = cudaSuccess;
+  for (int i = 0; i < n; i++) {
+    const cudaError_t e = cudaFree(idle[i]);
+    if (first == cudaSuccess) first = e;
+  }
+  if (count) *count = n;
+  return first;
+}
+
 }  // namespace
 
 cudaError_t host_workspace_take(size_t bytes, HostWorkspace &w) {
@@ -80,7 +106,14 @@ cudaError_t host_workspace_take(size_t bytes, HostWorkspace &w) {
     }
   }
   if (old) cudaFree(old);
-  e = cudaMalloc(&w.p, w.slot >= 0 ? want : bytes);
+  const size_t size = w.slot >= 0 ? want : bytes;
+  e = cudaMalloc(&w.p, size);
+  if (e == cudaErrorMemoryAllocation) {  // what lies idle here may be what is missing
+    int freed = 0;
+    release_idle(ctx, &freed);
+    cudaGetLastError();  // the next launch must not report this one
+    if (freed) e = cudaMalloc(&w.p, size);
+  }
   if (e != cudaSuccess) {
     if (w.slot >= 0) {
       std::lock_guard<std::mutex> lock(g_mutex);
@@ -107,17 +140,6 @@ void host_workspace_return(HostWorkspace &w, bool keep) {
   w = HostWorkspace{nullptr, -1};
 }
 
-int host_workspace_release_idle() {
-  const unsigned long long ctx = context_id();
-  int st = COGNI_QMM_OK;
-  std::lock_guard<std::mutex> lock(g_mutex);
-  for (Slot &s : g_slots) {
-    if (!s.bytes || s.lent || s.ctx != ctx) continue;
-    const cudaError_t e = cudaFree(s.p);
-    if (e != cudaSuccess && st == COGNI_QMM_OK) st = (int)e;
-    s = Slot{};
-  }
-  return st;
-}
+int host_workspace_release_idle() { return (int)release_idle(context_id(), nullptr); }
 
 }  // namespace cogni

@@ -169,15 +169,6 @@ void gemm_prefill_set_split(int mode);
 void gemm_prefill_set_stage_raw(int on);
 void gemm_prefill_set_pair(int on);
 
-// Device memory of the host-buffer call (host_workspace.cu), lent to one call at a time.
-struct HostWorkspace {
-  void *p;
-  int slot;  // -1: not kept
-};
-cudaError_t host_workspace_take(size_t bytes, HostWorkspace &w);
-void host_workspace_return(HostWorkspace &w, bool keep);
-int host_workspace_release_idle();
-
 // Kernel selection (dispatch.cu): picks the tiled kernel when the shape allows it, else the
 // general row-per-warp kernel.
 int launch_gemv(int type, const void *d_w, const float *d_x, const float *d_addend,

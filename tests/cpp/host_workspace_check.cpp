@@ -1,0 +1,107 @@
+// The memory that the host-buffer call keeps (csrc/host_workspace.cu), on a device that is made up: a
+// memory of fixed size whose blocks belong to the context that is current.
+#include <cuda.h>
+#include <cuda_runtime_api.h>
+#include <stdio.h>
+#include <string.h>
+
+#include <map>
+
+#include "../../cogni_ml_b200/csrc/host_workspace.cuh"
+
+namespace {
+
+const size_t kMB = (size_t)1 << 20;
+size_t capacity = (size_t)1 << 40, used = 0;
+unsigned long long current = 0, runtime_context = 1;  // 0: no context is current on this thread
+int mallocs = 0, bad_frees = 0;
+cudaError_t last_error = cudaSuccess;
+struct Block {
+  size_t bytes;
+  unsigned long long ctx;
+};
+std::map<void *, Block> blocks;
+char *next_address = reinterpret_cast<char *>((size_t)1 << 40);
+
+CUresult get_current(CUcontext *c) {
+  *c = reinterpret_cast<CUcontext>(current);
+  return CUDA_SUCCESS;
+}
+CUresult get_id(CUcontext c, unsigned long long *id) {
+  *id = 100 + reinterpret_cast<unsigned long long>(c);
+  return CUDA_SUCCESS;
+}
+
+int failures = 0;
+void expect(bool ok, const char *what) {
+  if (!ok) {
+    printf("failed: %s\n", what);
+    failures++;
+  }
+}
+bool call(size_t bytes) {  // a whole call
+  cogni::HostWorkspace w;
+  if (cogni::host_workspace_take(bytes, w) != cudaSuccess) return false;
+  cogni::host_workspace_return(w, true);
+  return true;
+}
+
+}  // namespace
+
+extern "C" {
+cudaError_t cudaFree(void *p) {
+  if (!current) current = runtime_context;
+  if (!p) return cudaSuccess;
+  auto it = blocks.find(p);
+  if (it == blocks.end() || it->second.ctx != current) {
+    bad_frees++;
+    return cudaErrorInvalidValue;
+  }
+  used -= it->second.bytes;
+  blocks.erase(it);
+  return cudaSuccess;
+}
+cudaError_t cudaMalloc(void **p, size_t bytes) {
+  if (!current) current = runtime_context;
+  mallocs++;
+  if (used + bytes > capacity) return last_error = cudaErrorMemoryAllocation;
+  used += bytes;
+  *p = next_address;
+  next_address += bytes;
+  blocks[*p] = Block{bytes, current};
+  return cudaSuccess;
+}
+cudaError_t cudaGetLastError(void) {
+  const cudaError_t e = last_error;
+  last_error = cudaSuccess;
+  return e;
+}
+cudaError_t cudaGetDriverEntryPoint(const char *name, void **f, unsigned long long, cudaDriverEntryPointQueryResult *q) {
+  *f = !strcmp(name, "cuCtxGetId") ? reinterpret_cast<void *>(get_id) : reinterpret_cast<void *>(get_current);
+  *q = cudaDriverEntryPointSuccess;
+  return cudaSuccess;
+}
+}
+
+int main(int argc, char **argv) {
+  const char *what = argc > 1 ? argv[1] : "";
+  if (!strcmp(what, "memory")) {  // the device has room for the call, but not beside the idle blocks
+    capacity = 300 * kMB;
+    cogni::HostWorkspace a, b;
+    expect(cogni::host_workspace_take(100 * kMB, a) == cudaSuccess, "first block");
+    expect(cogni::host_workspace_take(120 * kMB, b) == cudaSuccess, "second block");
+    cogni::host_workspace_return(a, true);
+    cogni::host_workspace_return(b, true);
+    expect(call(250 * kMB), "a call that fits the device without the idle blocks");
+    expect(last_error == cudaSuccess, "no error left for the next launch to report");
+    expect(!call(400 * kMB), "a call that does not fit the device");
+    expect(last_error == cudaSuccess, "no error left after a failed call");
+    expect(call(50 * kMB) && call(50 * kMB), "calls after it");
+  } else {
+    printf("unknown check %s\n", what);
+    return 2;
+  }
+  expect(bad_frees == 0, "no free of another context's or an unknown block");
+  if (!failures) printf("ok\n");
+  return failures ? 1 : 0;
+}
