@@ -3,8 +3,8 @@
 // A call needs one block for weights, activations, bias and outputs.  cudaMalloc + cudaFree of it cost
 // 0.7 ms at best and several where other work is in flight (cudaFree waits for the whole device),
 // against 0.55 ms for the copy of a 9.4 MB weight: blocks are therefore kept, up to kKeepBytes and
-// kSlots in all, and handed from call to call.  A block belongs to one call at a time (several
-// threads get several blocks) and to the CUDA context that it was allocated in; nothing of its content
+// kSlots in a CUDA context, and handed from call to call.  A block belongs to one call at a time (several
+// threads get several blocks) and to the context that it was allocated in; nothing of its content
 // is ever read by a later call.  cogni_qmm_release_host_workspaces gives the idle ones back, and so does
 // a call for which the device has no memory left.
 //
@@ -14,23 +14,29 @@
 
 #include <cuda.h>
 #include <mutex>
-
+#include <new>
 
 namespace cogni {
+
+// The entries form a list that only grows; one whose block has been given back is used again.  What a
+// destroyed context leaves behind is its entries alone, a few words of host memory: its blocks went with it,
+// they are never touched again (its id never comes back), and they count against no other context's limits.
+struct HostSlot {
+  void *p;
+  size_t bytes;  // 0: free entry
+  unsigned long long ctx;
+  bool lent;
+  HostSlot *next;
+};
+
 namespace {
 
 constexpr int kSlots = 8;
-constexpr size_t kKeepBytes = (size_t)256 << 20;  // idle and lent blocks of all contexts together
+constexpr size_t kKeepBytes = (size_t)256 << 20;  // idle and lent blocks of a context together
 constexpr size_t kGrain = (size_t)2 << 20;
 
-struct Slot {
-  void *p;
-  size_t bytes;
-  unsigned long long ctx;
-  bool lent;
-};
 std::mutex g_mutex;
-Slot g_slots[kSlots];
+HostSlot *g_slots = nullptr;
 
 // An id that no other context of the process ever has (a later context can reuse a handle); 0 if
 // there is none.
@@ -58,10 +64,10 @@ cudaError_t release_idle(unsigned long long ctx, int *count) {
   int n = 0;
   {
     std::lock_guard<std::mutex> lock(g_mutex);
-    for (Slot &s : g_slots)
-      if (s.bytes && !s.lent && s.ctx == ctx) {
-        idle[n++] = s.p;
-        s = Slot{};
+    for (HostSlot *s = g_slots; ctx && s; s = s->next)
+      if (s->bytes && !s->lent && s->ctx == ctx && n < kSlots) {
+        idle[n++] = s->p;
+        s->bytes = 0;
       }
   }
   cudaError_t first = cudaSuccess;
@@ -76,37 +82,51 @@ cudaError_t release_idle(unsigned long long ctx, int *count) {
 }  // namespace
 
 cudaError_t host_workspace_take(size_t bytes, HostWorkspace &w) {
-  w = HostWorkspace{nullptr, -1};
+  w = HostWorkspace{nullptr, nullptr};
   cudaError_t e = cudaFree(nullptr);  // the runtime's context, where none is current yet
   if (e != cudaSuccess) return e;
   const size_t want = (bytes + kGrain - 1) / kGrain * kGrain;
   const unsigned long long ctx = context_id();
   void *old = nullptr;  // too small a block that makes room for this one
-  {
+  if (ctx) {
     std::lock_guard<std::mutex> lock(g_mutex);
-    int fit = -1, small = -1, empty = -1;
+    HostSlot *fit = nullptr, *small = nullptr, *empty = nullptr;
     size_t held = 0;
-    for (int i = 0; i < kSlots; i++) {
-      const Slot &s = g_slots[i];
-      held += s.bytes;
-      if (!s.bytes) empty = i;
-      else if (!s.lent && s.ctx == ctx && s.bytes >= want && (fit < 0 || s.bytes < g_slots[fit].bytes)) fit = i;
-      else if (!s.lent && s.ctx == ctx && s.bytes < want) small = i;
+    int own = 0;
+    for (HostSlot *s = g_slots; s; s = s->next) {
+      if (!s->bytes) {
+        empty = s;
+      } else if (s->ctx == ctx) {
+        held += s->bytes;
+        own++;
+        if (s->lent) continue;
+        if (s->bytes < want) small = s;
+        else if (!fit || s->bytes < fit->bytes) fit = s;
+      }
     }
-    if (ctx && fit >= 0) {
-      g_slots[fit].lent = true;
-      w = HostWorkspace{g_slots[fit].p, fit};
+    if (fit) {
+      fit->lent = true;
+      w = HostWorkspace{fit->p, fit};
       return cudaSuccess;
     }
-    const int slot = small >= 0 ? small : empty;
-    if (ctx && slot >= 0 && held - g_slots[slot].bytes + want <= kKeepBytes) {
-      old = g_slots[slot].p;
-      g_slots[slot] = Slot{nullptr, want, ctx, true};  // reserved; the pointer is set on return
-      w.slot = slot;
+    if (held - (small ? small->bytes : 0) + want <= kKeepBytes && (small || own < kSlots)) {
+      HostSlot *slot = small ? small : empty;
+      if (!slot && (slot = new (std::nothrow) HostSlot{})) {
+        slot->next = g_slots;
+        g_slots = slot;
+      }
+      if (slot) {
+        if (small) old = small->p;
+        slot->p = nullptr;  // reserved; the pointer is set on return
+        slot->bytes = want;
+        slot->ctx = ctx;
+        slot->lent = true;
+        w.slot = slot;
+      }
     }
   }
   if (old) cudaFree(old);
-  const size_t size = w.slot >= 0 ? want : bytes;
+  const size_t size = w.slot ? want : bytes;
   e = cudaMalloc(&w.p, size);
   if (e == cudaErrorMemoryAllocation) {  // what lies idle here may be what is missing
     int freed = 0;
@@ -115,11 +135,11 @@ cudaError_t host_workspace_take(size_t bytes, HostWorkspace &w) {
     if (freed) e = cudaMalloc(&w.p, size);
   }
   if (e != cudaSuccess) {
-    if (w.slot >= 0) {
+    if (w.slot) {
       std::lock_guard<std::mutex> lock(g_mutex);
-      g_slots[w.slot] = Slot{};
+      w.slot->bytes = 0;
     }
-    w = HostWorkspace{nullptr, -1};
+    w = HostWorkspace{nullptr, nullptr};
   }
   return e;
 }
@@ -127,17 +147,17 @@ cudaError_t host_workspace_take(size_t bytes, HostWorkspace &w) {
 // keep = false: the call failed, its block is not lent again
 void host_workspace_return(HostWorkspace &w, bool keep) {
   if (!w.p) return;
-  if (w.slot >= 0) {
+  if (w.slot) {
     std::lock_guard<std::mutex> lock(g_mutex);
     if (keep) {
-      g_slots[w.slot].p = w.p;
-      g_slots[w.slot].lent = false;
+      w.slot->p = w.p;
+      w.slot->lent = false;
     } else {
-      g_slots[w.slot] = Slot{};
+      w.slot->bytes = 0;
     }
   }
-  if (w.slot < 0 || !keep) cudaFree(w.p);
-  w = HostWorkspace{nullptr, -1};
+  if (!w.slot || !keep) cudaFree(w.p);
+  w = HostWorkspace{nullptr, nullptr};
 }
 
 int host_workspace_release_idle() { return (int)release_idle(context_id(), nullptr); }

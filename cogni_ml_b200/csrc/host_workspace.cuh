@@ -6,9 +6,10 @@
 
 namespace cogni {
 
+struct HostSlot;
 struct HostWorkspace {
   void *p;
-  int slot;  // -1: not kept
+  HostSlot *slot;  // nullptr: not kept
 };
 cudaError_t host_workspace_take(size_t bytes, HostWorkspace &w);
 void host_workspace_return(HostWorkspace &w, bool keep);

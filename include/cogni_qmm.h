@@ -386,9 +386,9 @@ int cogni_qmm_matmul_add_host(const float *x, int rows, int in_dim, const void *
                               float *y);
 
 /*
- * The host-buffer form keeps the device memory of its calls (at most 256 MB of the process, one block
- * per call in flight) for later calls.  This gives the blocks that no call is using, of the current
- * context, back to the device.  (No counterpart in the reference.)
+ * The host-buffer form keeps the device memory of its calls for later ones (one block per call in
+ * flight; at most eight blocks and 256 MB of a CUDA context).  This gives the blocks of the current
+ * context that no call is using back to the device.  (No counterpart in the reference.)
  */
 int cogni_qmm_release_host_workspaces(void);
 

@@ -1,11 +1,12 @@
 // The memory that the host-buffer call keeps (csrc/host_workspace.cu), on a device that is made up: a
-// memory of fixed size whose blocks belong to the context that is current.
+// memory of fixed size whose blocks belong to the context that is current, and contexts that come and go.
 #include <cuda.h>
 #include <cuda_runtime_api.h>
 #include <stdio.h>
 #include <string.h>
 
 #include <map>
+#include <vector>
 
 #include "../../cogni_ml_b200/csrc/host_workspace.cuh"
 
@@ -30,6 +31,19 @@ CUresult get_current(CUcontext *c) {
 CUresult get_id(CUcontext c, unsigned long long *id) {
   *id = 100 + reinterpret_cast<unsigned long long>(c);
   return CUDA_SUCCESS;
+}
+
+void destroy_context() {  // with its memory; the next one that the runtime makes is another
+  for (auto it = blocks.begin(); it != blocks.end();) {
+    if (it->second.ctx == current) {
+      used -= it->second.bytes;
+      it = blocks.erase(it);
+    } else {
+      ++it;
+    }
+  }
+  current = 0;
+  runtime_context++;
 }
 
 int failures = 0;
@@ -97,6 +111,19 @@ int main(int argc, char **argv) {
     expect(!call(400 * kMB), "a call that does not fit the device");
     expect(last_error == cudaSuccess, "no error left after a failed call");
     expect(call(50 * kMB) && call(50 * kMB), "calls after it");
+  } else if (!strcmp(what, "contexts")) {  // blocks are kept in a context however many were destroyed before it
+    for (int i = 0; i < 40; i++) {
+      expect(call(40 * kMB), "first call of a context");
+      const int before = mallocs;
+      expect(call(40 * kMB) && call(30 * kMB) && mallocs == before, "later calls of the context allocate nothing");
+      destroy_context();
+    }
+    // several blocks at once, no more than eight and 256 MB of them kept
+    std::vector<cogni::HostWorkspace> ws(12);
+    for (auto &w : ws) expect(cogni::host_workspace_take(20 * kMB, w) == cudaSuccess, "one of twelve blocks");
+    for (auto &w : ws) cogni::host_workspace_return(w, true);
+    expect(blocks.size() == 8 && used == 160 * kMB, "eight blocks are kept");
+    expect(call(240 * kMB) && used <= 256 * kMB, "256 MB are kept");
   } else {
     printf("unknown check %s\n", what);
     return 2;

@@ -1,5 +1,5 @@
 """The device memory that host-buffer calls keep, on the CPU: csrc/host_workspace.cu against a made-up
-device (tests/cpp/host_workspace_check.cpp) that runs out of memory."""
+device (tests/cpp/host_workspace_check.cpp) that runs out of memory and whose contexts are destroyed."""
 import os
 import shutil
 import subprocess
@@ -24,7 +24,7 @@ def check(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["memory"])
+@pytest.mark.parametrize("what", ["memory", "contexts"])
 def test_kept_blocks(check, what):
     out = subprocess.run([str(check), what], capture_output=True, text=True)
     assert out.returncode == 0 and out.stdout.strip() == "ok", out.stdout + out.stderr
