@@ -160,6 +160,15 @@ void host_workspace_return(HostWorkspace &w, bool keep) {
   w = HostWorkspace{nullptr, nullptr};
 }
 
-int host_workspace_release_idle() { return (int)release_idle(context_id(), nullptr); }
+int host_workspace_release_idle() {
+  {
+    std::lock_guard<std::mutex> lock(g_mutex);
+    const HostSlot *s = g_slots;
+    while (s && !s->bytes) s = s->next;
+    if (!s) return 0;  // nothing is held: no context is made for this
+  }
+  cudaFree(nullptr);  // a thread without a context yet: the runtime's, as for a call
+  return (int)release_idle(context_id(), nullptr);
+}
 
 }  // namespace cogni

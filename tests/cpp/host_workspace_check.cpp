@@ -124,6 +124,11 @@ int main(int argc, char **argv) {
     for (auto &w : ws) cogni::host_workspace_return(w, true);
     expect(blocks.size() == 8 && used == 160 * kMB, "eight blocks are kept");
     expect(call(240 * kMB) && used <= 256 * kMB, "256 MB are kept");
+  } else if (!strcmp(what, "thread")) {  // a thread that has not used CUDA yet gives the idle blocks back
+    expect(cogni::host_workspace_release_idle() == 0 && !current, "no context is made where nothing is held");
+    expect(call(40 * kMB) && used == 40 * kMB, "a call keeps its block");
+    current = 0;
+    expect(cogni::host_workspace_release_idle() == 0 && used == 0, "the block is given back");
   } else {
     printf("unknown check %s\n", what);
     return 2;

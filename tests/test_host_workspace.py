@@ -24,7 +24,7 @@ def check(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["memory", "contexts"])
+@pytest.mark.parametrize("what", ["memory", "contexts", "thread"])
 def test_kept_blocks(check, what):
     out = subprocess.run([str(check), what], capture_output=True, text=True)
     assert out.returncode == 0 and out.stdout.strip() == "ok", out.stdout + out.stderr
