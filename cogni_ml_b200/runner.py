@@ -126,16 +126,6 @@ class QuantProjectionRunner:
                                                 device=self.device)
             self._host_out[p.name] = torch.empty(tokens, p.weight.out_dim,
                                                  dtype=torch.float32).pin_memory()
-        # Neighbouring projections of one type that share their input run as one launch (q, k, v; gate,
-        # up): a 1024-row projection alone leaves more than half of the SMs idle.
-        self._launches: List[List[Projection]] = []
-        for p in projections:
-            last = self._launches[-1][0] if self._launches else None
-            if (last is not None and p.source == last.source and p.weight.type == last.weight.type
-                    and not p.residual and not last.residual):
-                self._launches[-1].append(p)
-            else:
-                self._launches.append([p])
         self._facade = ResidentSequenceRunner(tokens, self._do_upload, self._do_reset,
                                               self._run_token, self._do_read, self._run_tokens)
 
@@ -205,10 +195,23 @@ class QuantProjectionRunner:
     def _input(self, name: str) -> torch.Tensor:
         return self._external.get(name, self._dev_in[name])
 
+    def _launch_groups(self) -> List[List[Projection]]:
+        """Neighbouring projections of one type that share their input run as one launch (q, k, v; gate,
+        up): a 1024-row projection alone leaves more than half of the SMs idle."""
+        groups: List[List[Projection]] = []
+        for p in self.projections:
+            last = groups[-1][0] if groups else None
+            if (last is not None and p.source == last.source and p.weight.type == last.weight.type
+                    and not p.residual and not last.residual):
+                groups[-1].append(p)
+            else:
+                groups.append([p])
+        return groups
+
     def _run_tokens(self, active_tokens: int) -> None:
         if not self._weights:
             raise RuntimeError("upload_weights must run before run_sequence")
-        for group in self._launches:
+        for group in self._launch_groups():
             p = group[0]
             x = self._input(p.source)[:active_tokens]
             outs = [self._dev_out[g.name][:active_tokens] for g in group]

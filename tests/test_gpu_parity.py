@@ -501,6 +501,45 @@ def test_runner_lifecycle_matches_oracle(cuda, oracle):
     runner.close()  # idempotent, as every close in the reference's driver binding
 
 
+@pytest.mark.parametrize("qtype,hidden", [(Q4_K, 1024), (Q8_0, 288)])  # 288: no launch takes several
+@pytest.mark.parametrize("tokens", [1, 5, 16])
+def test_runner_shares_launches(cuda, oracle, qtype, hidden, tokens):
+    """q, k, v and (on a device input) gate, up run as one launch each: every output against the oracle,
+    also for fewer active rows and for the projections that are left when some are dropped."""
+    rows = {"q": 520, "k": 70, "v": 64, "o": 520, "gate": 300, "up": 333}
+    src = {"q": "x", "k": "x", "v": "x", "o": "x", "gate": "mid", "up": "mid"}
+    ws = {n: QuantWeight(synth.make_weight(qtype, r, hidden, 83 + i, i), qtype, r, hidden) for i, (n, r) in enumerate(rows.items())}
+    xs = {n: synth.make_activation(tokens, hidden, 83, i) for i, n in enumerate(("x", "mid", "unused"))}
+    res = synth.make_activation(tokens, rows["o"], 83, 9)
+    ps = [Projection(n, ws[n], src[n], "res" if n == "o" else None) for n in rows]
+    runner = QuantProjectionRunner.from_weights(ps, tokens, {"x": xs["x"], "mid": xs["unused"], "res": res}, cuda)
+    runner.use_device_sequence_input("mid", torch.from_numpy(xs["mid"]).to(cuda))
+    refs = {n: oracle.matmul_add(xs[src[n]], tokens, hidden, ws[n].raw, qtype, rows[n], np.zeros(rows[n], np.float32)).reshape(tokens, -1)
+            for n in rows}
+    refs["o"] = refs["o"] + res
+    runner.upload_weights()
+    runner.reset_sequence()
+    for active in sorted({tokens, (tokens + 1) // 2}, reverse=True):
+        for n in rows:
+            runner.output_device_ptr(n).fill_(float("nan"))
+        runner.active_tokens = active
+        runner.run_sequence()
+        out = runner.read_outputs()
+        for n in rows:
+            assert_close(out[n], refs[n][:active], n)
+            assert bool(runner.output_device_ptr(n)[active:].isnan().all()), "rows that are not active stay as they are"
+    # the list of projections is what runs, at any time
+    runner.projections = [p for p in ps if p.name in ("k", "up")]
+    runner.output_device_ptr("q").fill_(7.0)
+    runner.output_device_ptr("k").fill_(float("nan"))
+    runner.upload_weights()
+    runner.run_sequence()
+    out = runner.read_outputs()
+    assert_close(out["k"], refs["k"][:active], "k alone")
+    assert (out["q"] == 7.0).all()
+    runner.close()
+
+
 @pytest.mark.parametrize("qtype,in_dim,slabs", [
     (Q4_K, 4096, 2), (Q4_K, 4096, 4), (Q5_K, 2048, 2), (Q6_K, 12288, 4), (Q6_K, 12288, 3),
     (Q6_K, 5120, 5), (Q8_0, 2048, 2), (IQ4_NL, 2048, 2), (Q6_K, 3072, 3),
