@@ -14,6 +14,9 @@
 #include "qmm_common.cuh"
 
 namespace cogni {
+
+extern int g_force_rowwarp;  // dispatch.cu
+
 namespace {
 
 constexpr int kWarpsPerCta = 8;
@@ -387,7 +390,7 @@ int run_gemv(const void *d_w, const float *d_x, const float *d_addend, int64_t a
     // 221 -> 259 us with one group of 5 / 8 against 3 + 3 / 4 + 4, IQ4_NL 196 -> 165 / 219 -> 191).
     const int most = batch > 4 && out_dim >= 4 * 148 * 8 ? (TYPE == kIQ4_NL ? 8 : 6) : 4;
     const int bg = (batch + most - 1) / most, nb = (batch + bg - 1) / bg;  // 5 rows: 3 + 3, 9: 3 + 3 + 3
-    if ((reinterpret_cast<uintptr_t>(d_x) & 15) == 0 && (long long)out_dim * bg <= 0x7fffffffLL) {
+    if (g_force_rowwarp == 0 && (reinterpret_cast<uintptr_t>(d_x) & 15) == 0 && (long long)out_dim * bg <= 0x7fffffffLL) {
       if (nb == 1) return run_blocks<TYPE, 1>(d_w, d_x, d_addend, addend_stride, d_y, in_dim, out_dim, batch, bg, s);
       if (nb == 2) return run_blocks<TYPE, 2>(d_w, d_x, d_addend, addend_stride, d_y, in_dim, out_dim, batch, bg, s);
       if (nb == 3) return run_blocks<TYPE, 3>(d_w, d_x, d_addend, addend_stride, d_y, in_dim, out_dim, batch, bg, s);

@@ -44,6 +44,26 @@ def test_gemv_of_whole_blocks(cuda, oracle, qtype, batch, out_dim, in_dim):
     assert np.abs(dw.gemv(xo).cpu().numpy() - ref).max() <= 1e-5 * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("qtype", [Q8_0, IQ4_NL])
+@pytest.mark.parametrize("batch", [1, 2, 5])
+def test_row_per_warp_kernel_on_request(cuda, oracle, engine, qtype, batch):
+    """Kernel choice 1 runs the row-per-warp kernel: the bits of a call whose x no other kernel takes."""
+    out_dim, in_dim = 301, 2976
+    w = synth.make_weight(qtype, out_dim, in_dim, seed=49, tensor_id=qtype)
+    x = synth.make_activation(batch, in_dim, seed=49)
+    dw = DeviceQuantWeight.upload(QuantWeight(w, qtype, out_dim, in_dim), cuda)
+    want = dw.gemv(aligned_at(x, 4, cuda).view(torch.float32).view(batch, in_dim))
+    xd = torch.from_numpy(x).to(cuda)
+    engine.lib.cogni_qmm_set_kernel_choice(1)
+    try:
+        assert torch.equal(dw.gemv(xd), want)
+    finally:
+        engine.lib.cogni_qmm_set_kernel_choice(0)
+    assert not torch.equal(dw.gemv(xd), want)  # the block kernel adds in another order
+    ref = oracle.matmul_add(x, batch, in_dim, w, qtype, out_dim, np.zeros(out_dim, np.float32)).reshape(batch, out_dim)
+    assert np.abs(want.cpu().numpy() - ref).max() <= 1e-5 * np.abs(ref).max()
+
+
 @pytest.mark.parametrize("qtype,out_dim,in_dim,slabs", [
     (Q8_0, 700, 2976, 0), (IQ4_NL, 700, 2976, 0), (Q8_0, 9001, 288, 0), (IQ4_NL, 9001, 288, 0),  # block kernel
     (Q4_K, 700, 1024, 0), (IQ4_NL, 700, 1024, 0), (Q4_K, 597, 4096, 4), (Q6_K, 597, 12288, 3)])  # tiled, K slabs
