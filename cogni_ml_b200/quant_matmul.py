@@ -71,7 +71,7 @@ class QuantWeight:
 
 
 def _stream_ptr(stream: Optional[torch.cuda.Stream]) -> int:
-    if stream is not None:
+    if stream:  # None and 0 both stand for the current stream
         return stream.cuda_stream
     # the handle alone: 0.1 us of a launch against 3.3 us for a torch.cuda.current_stream() object
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())

@@ -57,3 +57,18 @@ def test_quant_weight_checks_its_byte_count():
         QuantWeight(raw[:-1], synth.Q4_K, 4, 512)
     with pytest.raises(ValueError):
         QuantWeight(raw, synth.Q4_K, 4, 500)
+
+
+def test_no_stream_and_stream_zero_are_the_current_stream(monkeypatch):
+    import torch
+    from cogni_ml_b200 import quant_matmul
+
+    class Stream:
+        cuda_stream = 0x5000
+
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 3)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda device: 0x7000 + device, raising=False)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: type("S", (), {"cuda_stream": 0x7003})())
+    assert quant_matmul._stream_ptr(None) == 0x7003
+    assert quant_matmul._stream_ptr(0) == 0x7003
+    assert quant_matmul._stream_ptr(Stream()) == 0x5000
