@@ -1903,7 +1903,11 @@ bool make_plan_pair(int in_dim, int nb, int pair, Params &p, size_t &smem, bool 
   const bool v2 = TYPE == kQ6_K && !dense;  // Q6_K batch 1-2: no decode areas, 2 bytes of x per element and batch row
   const bool dense_int = dense && kDenseInt<TYPE>;  // scales unpacked in registers
   const size_t area_floats = v2 || dense_int ? 0 : dense ? (size_t)16 * dense_area_row(C::NG) : (size_t)pair * nb * Area<TYPE>::BATCH;
-  const size_t off_red = off;    off = al(off + (size_t)fold_bufs(nb) * ((nblk + pair - 1) / pair) * 8 * nb * 8);  // [tile buffer][item][g][batch] float2
+  // partial sums, [tile buffer][item][g][batch] float2; above batch 2 the norm's sums (a double per warp
+  // and row) go there first, which is more than a row of one superblock needs
+  const size_t red_bytes = (size_t)fold_bufs(nb) * ((nblk + pair - 1) / pair) * 8 * nb * 8;
+  const size_t norm_bytes = dense ? (size_t)consumer_warps(TYPE, pair, nb) * nb * 8 : 0;
+  const size_t off_red = off;    off = al(off + (red_bytes > norm_bytes ? red_bytes : norm_bytes));
   const size_t off_area = off;   off = al(off + (size_t)consumer_warps(TYPE, pair, nb) * area_floats * 4);
   const size_t off_sx = off;     off = al(off + (size_t)(dense_int ? nblk : ngroups) * nb * 4);
   const size_t off_xx = off;

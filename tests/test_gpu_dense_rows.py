@@ -11,7 +11,7 @@ import numpy as np
 import pytest
 import torch
 
-from cogni_ml_b200 import DeviceQuantWeight, QuantMatmul, QuantWeight, synth
+from cogni_ml_b200 import DeviceQuantWeight, QuantMatmul, QuantWeight, gemv_many, synth
 
 pytestmark = pytest.mark.gpu
 Q8_0, Q4_K, Q5_K, Q6_K, IQ4_NL = synth.Q8_0, synth.Q4_K, synth.Q5_K, synth.Q6_K, synth.IQ4_NL
@@ -39,6 +39,24 @@ def test_largest_group_sums(cuda, oracle, engine, qtype, batch, out_dim, in_dim)
         bound[4] += 2.0 ** -14 * np.abs(x[4]).max() * np.abs(deq).sum(1)
     assert (np.abs(y - ref) <= bound).all()
     assert engine.lib.cogni_qmm_wait_timeouts() == 0
+
+
+@pytest.mark.parametrize("qtype", TYPES)
+@pytest.mark.parametrize("batch", [3, 4, 5, 8])
+def test_fused_norm_of_one_superblock(cuda, oracle, qtype, batch):
+    """The shortest rows: the norm's per-warp sums need more room than the rows' partial sums.  Activations
+    are quantised in steps of 2^-14 of their superblock's largest, half a step each."""
+    out_dim, in_dim = 100, 256
+    w = synth.make_weight(qtype, out_dim, in_dim, seed=63, tensor_id=qtype)
+    x = 3 * synth.make_activation(batch, in_dim, seed=63)
+    wn = (1.0 + 0.1 * synth.make_activation(1, in_dim, seed=63, tensor_id=2)).ravel().astype(np.float32)
+    dw = DeviceQuantWeight.upload(QuantWeight(w, qtype, out_dim, in_dim), cuda)
+    y = gemv_many([dw], torch.from_numpy(x).to(cuda), norm_weight=torch.from_numpy(wn).to(cuda))[0].cpu().numpy()
+    xn = oracle.rmsnorm(x, wn, 1e-6)
+    ref = oracle.matmul_add(xn, batch, in_dim, w, qtype, out_dim, np.zeros(out_dim, np.float32)).reshape(batch, out_dim)
+    deq = np.abs(oracle.dequantize(qtype, w, out_dim * in_dim).reshape(out_dim, in_dim).astype(np.float64))
+    bound = 2.0 ** -14 * np.abs(xn).max(1)[:, None] * deq.sum(1)[None, :]
+    assert (np.abs(y - ref) <= bound).all()
 
 
 def test_host_calls_of_several_threads_and_sizes(cuda, oracle, engine):
