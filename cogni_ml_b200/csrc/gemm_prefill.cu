@@ -1508,7 +1508,7 @@ int launch_typed(const void *d_w, const void *d_x, void *d_y, int out_type, int 
                       : TYPE == kIQ4_NL ? TileTime{{6.8, 10.3, 17.8}, {0.59, 0.56, 0.62}}
                                         : TileTime{{6.5, 7.5, 14.0}, {0.45, 0.50, 0.65}};
   // Few row tiles against many SMs (short prompts, narrow matrices): the CTAs of a cluster take
-  // equal parts of K of a tile, at least two superblocks each, none empty.
+  // equal parts of K of a tile, two or more superblocks each; the last part takes what is left, at least one.
   const int nks = k_in / kBK;
   const int widths[3] = {128, 256, 512};
   int bn = 0, splits = 0;

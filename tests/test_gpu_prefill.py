@@ -68,8 +68,7 @@ def test_gemm_staged_superblocks(cuda, oracle, engine, tile, qtype, m, n, k):
     """Rows that are multiples of 16 bytes (Q4_K / Q5_K always, Q6_K when in_dim is a multiple of
     2048) are fetched by TMA into shared memory and expanded from there; rows beyond out_dim are
     zero-filled boxes.  The result must equal the direct-read path bit for bit (same expansion,
-    same MMA order; without a split along K, whose four-way form adds the partial tiles in an
-    order that depends on the number of dequant warps, which differs between the two paths)."""
+    same MMA order; without a split along K, which the two paths' tile times place differently)."""
     engine.lib.cogni_qmm_set_kernel_choice({128: 49, 256: 50, 512: 51}[tile])
     engine.lib.cogni_qmm_set_kernel_choice(53)
     try:
@@ -146,8 +145,8 @@ def test_gemm_last_row_tile_is_reproducible(cuda, engine, qtype, m, n, k):
 @pytest.mark.parametrize("qtype,m,n,k", [(Q6_K, 513, 128, 4096), (Q4_K, 300, 260, 4352),
                                          (Q5_K, 64, 128, 8192), (Q8_0, 200, 130, 4096)])
 def test_gemm_split_along_k(cuda, oracle, engine, tile, qtype, m, n, k):
-    """Two CTAs per tile, half of K each, partial tiles added onto a zeroed y (chosen by the host
-    when there are few row tiles for the SMs; forced here).  k = 4352 gives unequal halves."""
+    """Two CTAs of a cluster per tile, half of K each, at every tile width (chosen by the host when there
+    are few row tiles for the SMs; forced here).  k = 4352 gives unequal halves."""
     engine.lib.cogni_qmm_set_kernel_choice({128: 49, 256: 50, 512: 51}[tile])
     engine.lib.cogni_qmm_set_kernel_choice(54)
     try:
@@ -158,7 +157,7 @@ def test_gemm_split_along_k(cuda, oracle, engine, tile, qtype, m, n, k):
         engine.lib.cogni_qmm_set_kernel_choice(52)
     assert not np.isnan(y).any()
     assert np.abs(y - ref).max() <= 1e-4 * np.abs(ref).max()
-    assert np.array_equal(y, y2), "two addends commute: the split result must be reproducible"
+    assert np.array_equal(y, y2), "the split result must be reproducible"
     assert engine.lib.cogni_qmm_wait_timeouts() == 0
 
 
@@ -166,11 +165,9 @@ def test_gemm_split_along_k(cuda, oracle, engine, tile, qtype, m, n, k):
                                          (Q8_0, 530, 300, 4096), (Q5_K, 1000, 384, 8192),
                                          (Q6_K, 512, 1024, 12288), (IQ4_NL, 77, 200, 6144)])
 def test_gemm_four_ordered_splits(cuda, oracle, engine, qtype, m, n, k):
-    """Four CTAs per tile, a quarter of K each.  Four float addends do not commute, so the kernel
-    fixes the order: the tile's columns form four groups, split z adds its part of group
-    (z + t) mod 4 at step t, and a turn counter per (tile, group) admits the steps in order.  Every
-    launch must therefore give the same bits; y is not zeroed (the first part of a group is
-    stored), so the output buffer starts as NaN here.  k = 4352 gives unequal quarters."""
+    """Four CTAs of a cluster per tile, a quarter of K each; their partial tiles are added in the order of
+    the parts.  Every launch must therefore give the same bits; y is written once and whole, so the output
+    buffer starts as NaN here.  k = 4352 gives unequal quarters."""
     w = synth.make_weight(qtype, n, k, seed=31, tensor_id=qtype)
     dw = DeviceQuantWeight.upload(QuantWeight(w, qtype, n, k), cuda)
     x = bf16_round(synth.make_activation(m, k, seed=31))
@@ -193,15 +190,27 @@ def test_gemm_four_ordered_splits(cuda, oracle, engine, qtype, m, n, k):
     assert lib.cogni_qmm_wait_timeouts() == 0
 
 
+def split_runs(k, parts):
+    """Whether a split of k columns into `parts` is one the host may choose: parts of whole superblocks, two
+    or more of them, and something left for the last one."""
+    steps = k // 64
+    part = ((steps + parts - 1) // parts + 3) // 4 * 4
+    return part >= 8 and (parts - 1) * part < steps
+
+
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("split", [54, 59, 69])
 @pytest.mark.parametrize("qtype,m,n,k", [(Q4_K, 17, 130, 4096), (Q5_K, 129, 257, 4352), (Q6_K, 257, 150, 4096),
-                                         (Q6_K, 1, 37, 4352), (Q8_0, 600, 129, 4096), (IQ4_NL, 128, 512, 4096)])
+                                         (Q6_K, 1, 37, 4352), (Q8_0, 600, 129, 4096), (IQ4_NL, 128, 512, 4096),
+                                         (Q4_K, 300, 129, 3840), (Q6_K, 140, 70, 7936), (Q8_0, 5, 200, 3840)])
 def test_gemm_cluster_splits(cuda, oracle, engine, qtype, m, n, k, split, out_dtype):
     """Two, four and eight CTAs of a cluster per tile, their partial tiles summed through distributed
     shared memory: ragged tokens and rows (n not a multiple of 4 takes the scalar stores), unequal
-    parts, both output types.  f32: the additions' order only, 1e-4; bf16 on top: half a unit in the
+    parts (eight of 3840: seven of two superblocks and one of one; of 7936: seven of four and one of three),
+    both output types.  f32: the additions' order only, 1e-4; bf16 on top: half a unit in the
     last place of a result of eight significant bits, at most 2^-8 of it (762.1 -> 764 is 2^-8.6)."""
+    if not split_runs(k, {54: 2, 59: 4, 69: 8}[split]):
+        pytest.skip("this K has no such split: the automatic plan would run")
     engine.lib.cogni_qmm_set_kernel_choice(split)
     try:
         w, x, y, ref = run_case(cuda, oracle, qtype, m, n, k, seed=19, out_dtype=out_dtype)
@@ -211,6 +220,27 @@ def test_gemm_cluster_splits(cuda, oracle, engine, qtype, m, n, k, split, out_dt
     assert not np.isnan(y).any()
     assert np.abs(y - ref).max() <= tol * np.abs(ref).max()
     assert engine.lib.cogni_qmm_wait_timeouts() == 0
+
+
+@pytest.mark.parametrize("qtype,k", [(Q4_K, 3840), (Q6_K, 4096), (Q8_0, 7936)])
+def test_gemm_split_asked_for_is_the_split_that_runs(cuda, engine, qtype, k):
+    """One, two, four and eight parts add in different orders: on tiles of one width no two of them give
+    the same f32 bits, so a choice that fell back to another plan would show."""
+    m, n, choose = 70, 300, engine.lib.cogni_qmm_set_kernel_choice
+    dw = DeviceQuantWeight.upload(QuantWeight(synth.make_weight(qtype, n, k, seed=33, tensor_id=qtype), qtype, n, k), cuda)
+    xd = torch.from_numpy(synth.make_activation(m, k, seed=33)).to(cuda).bfloat16()
+    ys = []
+    choose(49)   # 128-token tiles
+    try:
+        for split in (53, 54, 59, 69):
+            choose(split)
+            ys.append(dw.gemm(xd))
+    finally:
+        choose(52)
+        choose(48)
+    for i in range(4):
+        for j in range(i):
+            assert not torch.equal(ys[i], ys[j]), f"plans {i} and {j}"
 
 
 @pytest.mark.parametrize("qtype,n,k", [(Q4_K, 1024, 4096), (Q6_K, 512, 12288), (Q8_0, 512, 4096),
