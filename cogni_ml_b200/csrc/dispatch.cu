@@ -2,7 +2,6 @@
 #include <climits>
 
 #include "qmm_common.cuh"
-#include "tma_pipe.cuh"
 
 namespace cogni {
 
@@ -104,10 +103,6 @@ __global__ void __launch_bounds__(kTop2Threads)
   const int b = blockIdx.y, part = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float *row = logits + (long long)b * out_dim;
   KeyPair p{LLONG_MIN, LLONG_MIN};
-  // launched while the GEMV that writes the logits still runs: its last CTA's end, not a launch, is
-  // what the first load waits for
-  pdl_wait_prior_grid();
-#pragma unroll 4
   for (int i = part * kTop2Threads + threadIdx.x; i < out_dim; i += nparts * kTop2Threads)
     pair_insert(p, top1_key(row[i], (uint32_t)(index_base + i)));
   auto block_merge = [&](KeyPair &q) {
@@ -181,19 +176,12 @@ int launch_gemv_top2(int type, const void *d_w, const float *d_x, int in_dim, in
                                logits + (long long)b0 * out_dim, in_dim, out_dim, nb, resident, s);
     if (st) return st;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(kTop2Threads);
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   for (int b0 = 0; b0 < batch; b0 += kTop2Rows) {
-    cfg.gridDim = dim3(nparts, batch - b0 < kTop2Rows ? batch - b0 : kTop2Rows);
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, top2_scan_kernel, (const float *)logits + (long long)b0 * out_dim, out_dim,
-                                             index_base, ctr, parts + (long long)b0 * nparts * 2, nparts, d_idx + 2 * b0,
-                                             d_val + 2 * b0, d_key ? d_key + 2 * b0 : nullptr);
+    const dim3 grid(nparts, batch - b0 < kTop2Rows ? batch - b0 : kTop2Rows);
+    top2_scan_kernel<<<grid, kTop2Threads, 0, s>>>(logits + (long long)b0 * out_dim, out_dim, index_base, ctr,
+                                                   parts + (long long)b0 * nparts * 2, nparts, d_idx + 2 * b0,
+                                                   d_val + 2 * b0, d_key ? d_key + 2 * b0 : nullptr);
+    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return (int)e;
   }
   return COGNI_QMM_OK;
