@@ -386,18 +386,31 @@ int run_blocks(const void *d_w, const float *d_x, const float *d_addend, int64_t
   return run_blocks_rows<TYPE, (NB > 4 ? 4 : NB), (NB > 4 ? 4 : 1)>(d_w, d_x, d_addend, addend_stride, d_y, in_dim, out_dim, batch, bgroups, s);
 }
 
+// Rows of so few blocks that the block kernel's reductions across lanes and warps cost more than the
+// row-per-warp kernel's passes over them (of four columns, or two).  Measured, us, row-per-warp / block:
+// Q8_0 600 x 192 at batch 1 2.11 / 2.24, 600 x 224 2.41 / 2.25; at batch 2 Q8_0 100 x 96 2.01 / 2.41, 100 x 128
+// 2.23 / 2.28, IQ4_NL 100 x 128 1.95 / 2.54; Q8_0 100 x 96 at batch 4 2.19 / 2.53, 100 x 128 2.68 / 2.66; 600 x 32
+// at batch 5 2.42 / 2.70.  On many rows the weights' bytes decide, and the block kernel's wider loads: IQ4_NL
+// 20000 x 32 at batch 1 3.73 / 4.52, 20000 x 96 4.98 / 4.65.
+bool short_rows(int type, int blocks, int out_dim, int batch) {
+  if (out_dim > (batch <= 2 || batch == 4 ? 5000 : 2500)) return batch <= 2 && blocks == 1;
+  if (batch <= 2) return blocks <= (type == kQ8_0 && batch == 2 ? 3 : 6);
+  return batch <= 8 && blocks * (batch == 4 ? 1 : 2) <= 3;
+}
+
 template <int TYPE>
 int run_gemv(const void *d_w, const float *d_x, const float *d_addend, int64_t addend_stride,
              float *d_y, int in_dim, int out_dim, int batch, cudaStream_t s) {
   const uint8_t *w = static_cast<const uint8_t *>(d_w);
   if constexpr (TYPE == kQ8_0 || TYPE == kIQ4_NL) {
-    // 16-byte loads of x: rows are whole 128-byte blocks, so its base decides
     // Up to four columns a CTA; on many rows the unpacked weights serve up to eight (Q8_0: six, its
     // weights take more registers until they are unpacked; 20000 x 10016 at batch 5 / 8: 166 -> 143 /
     // 221 -> 259 us with one group of 5 / 8 against 3 + 3 / 4 + 4, IQ4_NL 196 -> 165 / 219 -> 191).
     const int most = batch > 4 && out_dim >= 4 * 148 * 8 ? (TYPE == kIQ4_NL ? 8 : 6) : 4;
     const int bg = (batch + most - 1) / most, nb = (batch + bg - 1) / bg;  // 5 rows: 3 + 3, 9: 3 + 3 + 3
-    if (g_force_rowwarp == 0 && (reinterpret_cast<uintptr_t>(d_x) & 15) == 0 && (long long)out_dim * bg <= 0x7fffffffLL) {
+    // 16-byte loads of x: rows are whole 128-byte blocks, so its base decides
+    if (g_force_rowwarp == 0 && !short_rows(TYPE, in_dim / 32, out_dim, batch) &&
+        (reinterpret_cast<uintptr_t>(d_x) & 15) == 0 && (long long)out_dim * bg <= 0x7fffffffLL) {
       if (nb == 1) return run_blocks<TYPE, 1>(d_w, d_x, d_addend, addend_stride, d_y, in_dim, out_dim, batch, bg, s);
       if (nb == 2) return run_blocks<TYPE, 2>(d_w, d_x, d_addend, addend_stride, d_y, in_dim, out_dim, batch, bg, s);
       if (nb == 3) return run_blocks<TYPE, 3>(d_w, d_x, d_addend, addend_stride, d_y, in_dim, out_dim, batch, bg, s);

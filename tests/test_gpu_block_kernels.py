@@ -64,6 +64,30 @@ def test_row_per_warp_kernel_on_request(cuda, oracle, engine, qtype, batch):
     assert np.abs(want.cpu().numpy() - ref).max() <= 1e-5 * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("qtype,batch,out_dim,longest", [
+    (Q8_0, 1, 37, 6), (IQ4_NL, 1, 5000, 6), (Q8_0, 2, 300, 3), (IQ4_NL, 2, 300, 6), (Q8_0, 4, 37, 3), (IQ4_NL, 7, 300, 1),
+    (Q8_0, 9, 37, 0), (IQ4_NL, 1, 5001, 1), (Q8_0, 2, 5001, 1), (Q8_0, 3, 5001, 0)])
+def test_short_rows_and_where_they_end(cuda, oracle, engine, qtype, batch, out_dim, longest):
+    """Rows of up to `longest` blocks run on the row-per-warp kernel, the next longer ones do not; both
+    against the oracle, with the tolerance of test_gemv_of_whole_blocks."""
+    choose = engine.lib.cogni_qmm_set_kernel_choice
+    for blocks in {1, longest, longest + 1} - {0}:
+        in_dim = 32 * blocks
+        w = synth.make_weight(qtype, out_dim, in_dim, seed=53, tensor_id=qtype)
+        x = synth.make_activation(batch, in_dim, seed=53)
+        dw = DeviceQuantWeight.upload(QuantWeight(w, qtype, out_dim, in_dim), cuda)
+        xd = torch.from_numpy(x).to(cuda)
+        y = dw.gemv(xd)
+        choose(1)
+        try:
+            row_per_warp = torch.equal(y, dw.gemv(xd))
+        finally:
+            choose(0)
+        assert row_per_warp == (blocks <= longest), f"{blocks} blocks"
+        ref = oracle.matmul_add(x, batch, in_dim, w, qtype, out_dim, np.zeros(out_dim, np.float32)).reshape(batch, out_dim)
+        assert np.abs(y.cpu().numpy() - ref).max() <= 1e-5 * np.abs(ref).max()
+
+
 @pytest.mark.parametrize("qtype,out_dim,in_dim,slabs", [
     (Q8_0, 700, 2976, 0), (IQ4_NL, 700, 2976, 0), (Q8_0, 9001, 288, 0), (IQ4_NL, 9001, 288, 0),  # block kernel
     (Q4_K, 700, 1024, 0), (IQ4_NL, 700, 1024, 0), (Q4_K, 597, 4096, 4), (Q6_K, 597, 12288, 3)])  # tiled, K slabs
