@@ -89,8 +89,8 @@ __device__ __forceinline__ void expand_block<kQ6_K>(const uint8_t *b, float *y, 
   }
 }
 
-// Any 2-byte aligned weights, any 4-byte aligned output: one warp per block, lane l writes element l
-// of every 32-wide group.
+// Any 2-byte aligned weights, any 4-byte aligned output, and small tensors: one warp per block, lane l
+// writes element l of every 32-wide group.
 template <int TYPE>
 __global__ void __launch_bounds__(256) dequantize_blocks_kernel(const uint8_t *__restrict__ w,
                                                                 float *__restrict__ out,
@@ -232,11 +232,19 @@ int run_embedding(const void *d_table, const int32_t *d_ids, int n_tokens, int v
   return (int)cudaGetLastError();
 }
 
+// Elements from which the 16-byte stores pay: below, their few CTAs each expand a chain of blocks while SMs
+// idle, and a warp per block is done first.  Measured, us, warp per block / 16-byte stores (graph replay):
+// Q8_0 64 K 1.77 / 2.40, 256 K 2.53 / 2.54, 512 K 3.32 / 2.43; IQ4_NL 128 K 2.07 / 2.14, 256 K 2.49 / 2.16; Q4_K 256 K
+// 1.93 / 2.80, 1.5 M 3.02 / 2.97; Q5_K 256 K 1.96 / 2.91, 2 M 3.49 / 3.69, 3 M 5.49 / 5.13; Q6_K 256 K 1.92 / 2.52, 2 M
+// 3.74 / 3.75, 3 M 4.92 / 4.81.
+template <int TYPE>
+constexpr int64_t kQuadsFrom = TYPE == kQ8_0 ? 1 << 18 : TYPE == kIQ4_NL ? 3 << 16 : TYPE == kQ4_K ? 3 << 19 : 3 << 20;
+
 template <int TYPE>
 int run(const void *d_w, int64_t n, float *d_out, cudaStream_t s) {
   long long nblocks = n / BlockGeom<TYPE>::elems;
   if (nblocks == 0) return COGNI_QMM_OK;
-  if (((reinterpret_cast<uintptr_t>(d_w) | reinterpret_cast<uintptr_t>(d_out)) & 15) == 0) {
+  if (n >= kQuadsFrom<TYPE> && ((reinterpret_cast<uintptr_t>(d_w) | reinterpret_cast<uintptr_t>(d_out)) & 15) == 0) {
     constexpr int per_cta = 256 / kQuadLanes<TYPE> * kQuadUnroll<TYPE>;
     const long long ctas = (nblocks + per_cta - 1) / per_cta;
     if (ctas <= 0x7fffffffLL) {

@@ -111,6 +111,24 @@ def test_residual_in_place(cuda, engine, qtype, out_dim, in_dim, slabs):
         engine.lib.cogni_qmm_set_kernel_choice(60)
 
 
+@pytest.mark.parametrize("qtype,elements", [(Q8_0, 1 << 18), (IQ4_NL, 3 << 16), (Q4_K, 3 << 19), (Q5_K, 3 << 20), (Q6_K, 3 << 20)])
+@pytest.mark.parametrize("more", [-1, 0, 1, 33, 129])
+@pytest.mark.parametrize("w_at,y_at", [(0, 0), (2, 0), (0, 4)])
+def test_dequantize_from_where_the_wide_stores_begin(cuda, oracle, engine, qtype, elements, more, w_at, y_at):
+    """The same at the sizes from which a tensor takes the 16-byte stores: whole CTAs of them, and remainders
+    of one block and more."""
+    n = elements + more * (32 if qtype in (Q8_0, IQ4_NL) else 256)
+    w = synth.make_weight(qtype, 1, n, seed=45, tensor_id=qtype)
+    raw = aligned_at(w, w_at, cuda)
+    buf = torch.full((n + 8,), 7.0, device=cuda)
+    start = (-buf.data_ptr()) % 16 // 4 + y_at // 4
+    out = buf[start:start + n]
+    st = engine.lib.cogni_qmm_dequantize(qtype, raw.data_ptr(), n, out.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    assert st == 0
+    assert np.array_equal(out.cpu().numpy().view(np.uint32), oracle.dequantize(qtype, w, n).view(np.uint32))
+    assert buf[:start].eq(7.0).all() and buf[start + n:].eq(7.0).all()
+
+
 @pytest.mark.parametrize("qtype", [Q8_0, Q4_K, Q5_K, Q6_K, IQ4_NL])
 @pytest.mark.parametrize("blocks", [1, 7, 33, 129])
 @pytest.mark.parametrize("w_at,y_at", [(0, 0), (2, 0), (0, 4)])
