@@ -90,12 +90,12 @@ int cogni_qmm_set_kernel_choice(int choice) {
     gemm_prefill_set_pair(choice == 57);
     return COGNI_QMM_OK;
   }
-  if (choice >= 52 && choice <= 54) {  // prefill split along K: automatic / never / two splits wherever allowed
+  if (choice >= 52 && choice <= 54) {  // prefill split along K: automatic / never / two parts wherever allowed
     gemm_prefill_set_split(choice - 52);
     return COGNI_QMM_OK;
   }
-  if (choice == 59 || choice == 69) {  // prefill split along K: four / eight parts wherever allowed
-    gemm_prefill_set_split(choice == 59 ? 3 : 4);
+  if (choice == 59 || choice == 69 || choice == 70) {  // the same: four / eight / three parts wherever allowed
+    gemm_prefill_set_split(choice == 59 ? 4 : choice == 69 ? 8 : 3);
     return COGNI_QMM_OK;
   }
   if (choice >= 27 && choice <= 30) {  // at least 1 .. 4 column ranges per row of the tiled GEMV

@@ -1305,7 +1305,7 @@ EncodeTiledFn encode_tiled_fn() {
 
 int g_prefill_force_bn = 0;  // diagnostics: 0 = automatic, else the token-tile width to use
 int g_prefill_stage_raw = 1;    // diagnostics: 0 = dequant threads read global memory directly
-int g_prefill_force_split = 0;  // diagnostics: 0 = automatic, 1 = never split along K, 2 / 3 / 4 = two / four / eight splits where allowed
+int g_prefill_force_split = 0;  // diagnostics: 0 = automatic, 1 = never split along K, else that many parts where allowed
 
 // k-steps of a part of an n-way split: whole superblocks
 int ksteps_per_split(int nks, int splits) { return splits > 1 ? ((nks + splits - 1) / splits + 3) / 4 * 4 : nks; }
@@ -1343,9 +1343,9 @@ void split_launch_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &attr, dim
 // How many clusters of `splits` CTAs run at once (every instance takes a whole SM's shared memory,
 // so the narrowest one stands for all).
 int split_capacity(int dev, int splits) {
-  static std::atomic<int> cached[64][4];  // for 2, 4, 8 CTAs: 1 + the count
+  static std::atomic<int> cached[64][9];  // 1 + the count
   if (dev < 0 || dev >= 64) return 0;
-  std::atomic<int> &slot = cached[dev][splits == 2 ? 1 : splits == 4 ? 2 : 3];
+  std::atomic<int> &slot = cached[dev][splits];
   int v = slot.load();
   if (v == 0) {
     cudaLaunchConfig_t cfg;
@@ -1479,13 +1479,16 @@ template <int TYPE>
 int launch_typed(const void *d_w, const void *d_x, void *d_y, int out_type, int m_rows, int n_out,
                  int k_in, cudaStream_t s) {
   // Token-tile width and split along K: wider tiles do less dequant work per flop, narrower ones and
-  // splits fill the SMs.  A wave of tiles of 128 / 256 / 512 tokens takes fixed + step x k-steps
-  // (us, fitted to measured launches of one wave with 16 to 192 k-steps; Q6_K rows that TMA cannot
-  // describe are read by the dequant threads and take twice as long), a split adds the exchange of
-  // the partial tiles.  The plan with the least waves x time is taken.  Measured against the whole-K
-  // plans it replaces (us): Q5_K 77 x 4096 x 4096 (m, n, k) 28.3 -> 14.7 (128 tokens, four parts),
-  // Q4_K 20 x 1024 x 4096 19.8 -> 9.2 (eight), Q4_K 300 x 4096 x 4096 32 -> 24.6 (two), Q6_K
-  // 512 x 4096 x 12288 62 -> 55 (four, 512 tokens: atomic turn-taking through global memory before).
+  // splits fill the SMs.  A wave of tiles of 128 / 256 / 512 tokens takes fixed + step x k-steps (a little less
+  // where a part of the tile is empty), a split adds the exchange of the partial tiles, per token column; the
+  // plan with the least waves x time is taken.
+  // The constants (us) are fitted so that this is the fastest plan, over every plan's time on shapes of 17 to
+  // 6000 tokens, 256 to 16384 rows and 1024 to 12288 columns; on 3555 of them the plan taken is 0.3 % slower than
+  // the fastest on average.  (Times fitted to single waves chose worse: several waves of 512-token tiles take
+  // longer than as many single ones, Q8_0 1800 x 5120 x 5120 (m, n, k) 187 us whole, 149 in two parts.)
+  // Three parts are for 34 to 45 tiles: 33 clusters of four fit the GPU at once, 45 of three (Q8_0
+  // 694 x 2184 x 4864 49 -> 41.6).  Against whole K (us): Q5_K 77 x 4096 x 4096 28.3 -> 14.7 (128 tokens, four
+  // parts), Q4_K 20 x 1024 x 4096 19.8 -> 9.2 (eight), Q4_K 300 x 4096 x 4096 32 -> 24.6 (two).
   static int sms_of[64] = {0};  // per device: a process may drive GPUs of different sizes
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1501,12 +1504,12 @@ int launch_typed(const void *d_w, const void *d_x, void *d_y, int out_type, int 
   // of a matrix with at least one full row tile can be fetched by TMA: the raw superblocks of the
   // tile's rows are then staged through shared memory
   const bool staged = TYPE != kQ8_0 && row_bytes % 16 == 0 && n_out >= kBM && g_prefill_stage_raw;
-  struct TileTime { double fixed[3], step[3]; };
-  const TileTime tt = TYPE == kQ6_K ? (staged ? TileTime{{6.5, 10.0, 13.0}, {0.62, 0.62, 0.72}}
-                                              : TileTime{{4.0, 8.0, 13.0}, {1.15, 1.30, 1.30}})
-                      : TYPE == kQ8_0   ? TileTime{{5.5, 10.0, 17.5}, {0.76, 0.76, 0.72}}
-                      : TYPE == kIQ4_NL ? TileTime{{6.8, 10.3, 17.8}, {0.59, 0.56, 0.62}}
-                                        : TileTime{{6.5, 7.5, 14.0}, {0.45, 0.50, 0.65}};
+  struct TileTime { double fixed[3], step[3], column, empty; };
+  const TileTime tt = TYPE == kQ6_K ? (staged ? TileTime{{4.40, 5.18, 9.59}, {0.70, 0.79, 0.85}, 0.008, 0.18}
+                                              : TileTime{{3.70, 7.22, 7.09}, {1.38, 1.40, 1.57}, 0.011, 0.0})
+                      : TYPE == kQ8_0   ? TileTime{{4.95, 2.52, 11.42}, {0.79, 1.10, 1.02}, 0.005, 0.0}
+                      : TYPE == kIQ4_NL ? TileTime{{5.05, 5.85, 9.13}, {0.58, 0.65, 0.78}, 0.008, 0.156}
+                                        : TileTime{{5.35, 6.31, 12.94}, {0.49, 0.53, 0.70}, 0.006, 0.0};
   // Few row tiles against many SMs (short prompts, narrow matrices): the CTAs of a cluster take
   // equal parts of K of a tile, two or more superblocks each; the last part takes what is left, at least one.
   const int nks = k_in / kBK;
@@ -1515,16 +1518,20 @@ int launch_typed(const void *d_w, const void *d_x, void *d_y, int out_type, int 
   double best = 1e30;
   for (int i = 0; i < 3; i++) {
     if (g_prefill_force_bn && g_prefill_force_bn != widths[i]) continue;
-    for (int sp = 1; sp <= 8; sp *= 2) {
+    for (int sp : {1, 2, 3, 4, 8}) {
       const int per = ksteps_per_split(nks, sp);
       if (sp > 1 && (per < 8 || (sp - 1) * per >= nks || g_prefill_force_split == 1)) continue;
+      // Q8_0's direct loads contend where three parts fill the SMs with tiles narrower than the tokens (229 x
+      // 2760 x 5376: 128 tokens in three parts 33.7 us, 256 in four on two thirds of the SMs 26.8)
+      if (sp == 3 && TYPE == kQ8_0 && widths[i] != 512 && m_rows > widths[i] && g_prefill_force_split != 3) continue;
       const int at_once = sp == 1 ? sms : split_capacity(dev, sp);
       if (at_once == 0) continue;
       const long long tiles = row_tiles * ((m_rows + widths[i] - 1) / widths[i]);
-      double t = tt.fixed[i] + tt.step[i] * per;
-      if (sp > 1) t += 1.0 + 0.01 * (m_rows < widths[i] ? m_rows : widths[i]);
+      const int tokens = m_rows < widths[i] ? m_rows : widths[i];
+      double t = tt.fixed[i] + tt.step[i] * per * (1.0 - tt.empty * (widths[i] - tokens) / widths[i]);
+      if (sp > 1) t += tt.column * tokens;
       double c = (double)((tiles + at_once - 1) / at_once) * t;
-      if (g_prefill_force_split >= 2 && sp == 1 << (g_prefill_force_split - 1)) c -= 1e6;
+      if (g_prefill_force_split >= 2 && sp == g_prefill_force_split) c -= 1e6;
       if (c < best) { best = c; bn = widths[i]; splits = sp; }
     }
   }

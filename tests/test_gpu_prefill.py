@@ -199,17 +199,17 @@ def split_runs(k, parts):
 
 
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("split", [54, 59, 69])
+@pytest.mark.parametrize("split", [54, 59, 69, 70])
 @pytest.mark.parametrize("qtype,m,n,k", [(Q4_K, 17, 130, 4096), (Q5_K, 129, 257, 4352), (Q6_K, 257, 150, 4096),
                                          (Q6_K, 1, 37, 4352), (Q8_0, 600, 129, 4096), (IQ4_NL, 128, 512, 4096),
                                          (Q4_K, 300, 129, 3840), (Q6_K, 140, 70, 7936), (Q8_0, 5, 200, 3840)])
 def test_gemm_cluster_splits(cuda, oracle, engine, qtype, m, n, k, split, out_dtype):
-    """Two, four and eight CTAs of a cluster per tile, their partial tiles summed through distributed
+    """Two, three, four and eight CTAs of a cluster per tile, their partial tiles summed through distributed
     shared memory: ragged tokens and rows (n not a multiple of 4 takes the scalar stores), unequal
     parts (eight of 3840: seven of two superblocks and one of one; of 7936: seven of four and one of three),
     both output types.  f32: the additions' order only, 1e-4; bf16 on top: half a unit in the
     last place of a result of eight significant bits, at most 2^-8 of it (762.1 -> 764 is 2^-8.6)."""
-    if not split_runs(k, {54: 2, 59: 4, 69: 8}[split]):
+    if not split_runs(k, {54: 2, 59: 4, 69: 8, 70: 3}[split]):
         pytest.skip("this K has no such split: the automatic plan would run")
     engine.lib.cogni_qmm_set_kernel_choice(split)
     try:
@@ -224,7 +224,7 @@ def test_gemm_cluster_splits(cuda, oracle, engine, qtype, m, n, k, split, out_dt
 
 @pytest.mark.parametrize("qtype,k", [(Q4_K, 3840), (Q6_K, 4096), (Q8_0, 7936)])
 def test_gemm_split_asked_for_is_the_split_that_runs(cuda, engine, qtype, k):
-    """One, two, four and eight parts add in different orders: on tiles of one width no two of them give
+    """One, two, three, four and eight parts add in different orders: on tiles of one width no two of them give
     the same f32 bits, so a choice that fell back to another plan would show."""
     m, n, choose = 70, 300, engine.lib.cogni_qmm_set_kernel_choice
     dw = DeviceQuantWeight.upload(QuantWeight(synth.make_weight(qtype, n, k, seed=33, tensor_id=qtype), qtype, n, k), cuda)
@@ -232,13 +232,13 @@ def test_gemm_split_asked_for_is_the_split_that_runs(cuda, engine, qtype, k):
     ys = []
     choose(49)   # 128-token tiles
     try:
-        for split in (53, 54, 59, 69):
+        for split in (53, 54, 70, 59, 69):
             choose(split)
             ys.append(dw.gemm(xd))
     finally:
         choose(52)
         choose(48)
-    for i in range(4):
+    for i in range(5):
         for j in range(i):
             assert not torch.equal(ys[i], ys[j]), f"plans {i} and {j}"
 
