@@ -1019,7 +1019,7 @@ template <int TYPE> constexpr bool kDenseInt = TYPE == kQ4_K || TYPE == kQ5_K ||
 // leaves 25 KB more of it to the stages.  With the quantiser's wide stores, batch 8, us, before -> now:
 // Q4_K 12288 x 4096 16.3 -> 13.9, 34816 x 5120 57.3 -> 47.6; Q5_K 12288 x 4096 17.8 -> 15.2; Q6_K 12288 x
 // 4096 23.8 -> 19.5, 4096 x 4096 12.9 -> 10.1, 151936 x 4096 182 -> 152 (3.4 TB/s), and the 151936 x
-// 5120 head with its top-1 316 -> 181 (three stages fit now, two before).  Bound by the consumer warps:
+// 5120 head with its top-1 316 -> 181 (three stages fit now, two before; 175 with twenty consumer warps).  Bound by the consumer warps:
 // 16 MMAs, 64 integer multiply-adds and 48 unpacking instructions a superblock are its core.
 //
 // MMAs of one superblock for all NB batch rows.  xg: this lane's B fragments of the superblock's
@@ -2102,9 +2102,9 @@ int choose_slabs(int in_dim, int nbk, int tiles, bool thin, bool workspace_ok) {
   const int nblk = in_dim / 256, sms = sm_count();
   int best = 0;
   float best_cost = 0.f;
-  // Where whole rows fit, slabs are correct but not faster: the fence and the ticket of every tile
-  // part sit in a consumer warp's path (measured on the 9B FFN: 15.1 against 13.2 us for ffn_down
-  // with four slabs), so such a launch only uses them when asked to.  Where a row of activations
+  // Where whole rows fit, slabs are correct but not faster: the ticket and the read-back of every tile
+  // part sit in a consumer warp's path (Q6_K 4096 x 12288 at batch 1: 14.0 us with four slabs, 14.3 with two,
+  // against 12.3; Q4_K 4096 x 4096 6.2 with two against 4.8), so such a launch only uses them when asked to.  Where a row of activations
   // does not fit shared memory, slabs replace the column ranges (one launch instead of several).
   Params whole{};
   size_t whole_smem = 0;
