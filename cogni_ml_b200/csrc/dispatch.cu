@@ -103,6 +103,7 @@ __global__ void __launch_bounds__(kTop2Threads)
   const int b = blockIdx.y, part = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float *row = logits + (long long)b * out_dim;
   KeyPair p{LLONG_MIN, LLONG_MIN};
+#pragma unroll 4  // a thread's eight loads in two batches
   for (int i = part * kTop2Threads + threadIdx.x; i < out_dim; i += nparts * kTop2Threads)
     pair_insert(p, top1_key(row[i], (uint32_t)(index_base + i)));
   auto block_merge = [&](KeyPair &q) {
